@@ -992,8 +992,7 @@ int lbm_create(const lbm_params* pin, lbm_sim** out) {
   for (int k = 0; k < 3; ++k) m.w_init[k] = p.w_init[k];
   // rates at the uniform omega, ComputeRelaxation_MRT (C1:1029-1048, C6:1002-1021)
   const double oq = m.q_of_omega ? 8. * (2. - omega) / (8. - omega) : p.s_q;
-  const double S_uni[9] = {0.0, p.s_e, p.s_eps, 0.0, oq, 0.0, oq, omega, omega};
-  for (int k = 0; k < 9; ++k) m.S_uni[k] = S_uni[k];
+  m.sq_uni = oq;
   static const double w[9] = {4.0 / 9, 1.0 / 9, 1.0 / 9, 1.0 / 9, 1.0 / 9,
                               1.0 / 36, 1.0 / 36, 1.0 / 36, 1.0 / 36};
   for (int k = 0; k < 9; ++k) m.shift_f[k] = (float)(p.rho0 * w[k] * (36.0 * p.d_mrt - 1.0));

@@ -113,7 +113,7 @@ struct Model {
   double rho0, nu, omega, s_e, s_eps, s_q, d_mrt, pi, zeta;
   double tau_y, m_pap, gamma_min;
   double w_init[3];
-  double S_uni[9];   // rates at the uniform omega (Newtonian nodes)
+  double sq_uni;     // s_q at the uniform omega (Newtonian nodes)
   // FP32 copies, so kernels never convert per node
   float rho0_f, nu_f, d_mrt_f, pi_f, zeta_f, tau_y_f, m_pap_f, gamma_min_f;
   float s_e_f, s_eps_f, sq_uni_f, omega_f;

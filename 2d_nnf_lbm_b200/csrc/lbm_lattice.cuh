@@ -150,13 +150,6 @@ __device__ __forceinline__ void edge_equilibrium(const LatticeArgs& a, int i, in
   for (int k = 0; k < 9; ++k) f[k] = (T)h[k];
 }
 
-// ComputeRelaxation_MRT (C1:1029-1048 fixed q; C6:1002-1021 q of omega).
-__device__ __forceinline__ void rates_double(const Model& m, double omega, double* S) {
-  const double oq = m.q_of_omega ? 8. * (2. - omega) / (8. - omega) : m.s_q;
-  S[0] = 0.0; S[1] = m.s_e; S[2] = m.s_eps; S[3] = 0.0;
-  S[4] = oq; S[5] = 0.0; S[6] = oq; S[7] = omega; S[8] = omega;
-}
-
 // ---------------------------------------------------------------------------
 // SPM solid fraction of one node for one disk (C1:464-476).
 __device__ __forceinline__ double phi_double(double di, double dj, double R, double zeta,
@@ -185,156 +178,160 @@ __device__ __forceinline__ float phi_float(float di, float dj, float R, float ze
 }
 
 // ---------------------------------------------------------------------------
-// Collision_MRT for one node in plain FP64 (C1:886-921; Chai strain rate and
-// Papanastasiou viscosity C6:903-958).  Same operations, same order as the
-// reference.  Returns the new omega and writes stress / yield code.
+// Stress, yield code and omega a collision leaves for the next one.
 struct NodeOut {
   double t11, t22, t12, omega;
   int yield;
 };
 
-__device__ __forceinline__ void collide_double(const Model& m, double* f, double RHO, double UX,
-                                               double UY, double GX, double GY, const double* S,
-                                               bool want_stress, NodeOut& no) {
-  const double d_mrt = m.d_mrt;
-  const double f0 = f[0], f1 = f[1], f2 = f[2], f3 = f[3], f4 = f[4], f5 = f[5], f6 = f[6],
-               f7 = f[7], f8 = f[8];
-  double M[9], MF[9], MEQ[9];
-  M[0] = f0 + f1 + f2 + f3 + f4 + f5 + f6 + f7 + f8;
-  M[1] = -4.0 * f0 - f1 - f2 - f3 - f4 + 2.0 * (f5 + f6 + f7 + f8);
-  M[2] = 4.0 * f0 - 2.0 * (f1 + f2 + f3 + f4) + (f5 + f6 + f7 + f8);
-  M[3] = f1 - f3 + f5 - f6 - f7 + f8;
-  M[4] = -2.0 * (f1 - f3) + f5 - f6 - f7 + f8;
-  M[5] = f2 - f4 + f5 + f6 - f7 - f8;
-  M[6] = -2.0 * (f2 - f4) + f5 + f6 - f7 - f8;
-  M[7] = f1 - f2 + f3 - f4;
-  M[8] = f5 - f6 + f7 - f8;
-  const double F_X = RHO * (GX + 0.0), F_Y = RHO * (GY + 0.0);
-  MF[0] = 0.0;
-  MF[1] = 6.0 * (F_X * UX + F_Y * UY);
-  MF[2] = -6.0 * (F_X * UX + F_Y * UY);
-  MF[3] = F_X;
-  MF[4] = -F_X;
-  MF[5] = F_Y;
-  MF[6] = -F_Y;
-  MF[7] = 2.0 * (F_X * UX - F_Y * UY);
-  MF[8] = F_Y * UX + F_X * UY;
-  const double U2 = UX * UX + UY * UY;
-  MEQ[0] = RHO;
-  MEQ[1] = RHO * (-2.0 + 3. * U2);
-  MEQ[2] = RHO * (1.0 - 3. * U2);
-  MEQ[3] = RHO * (UX);
-  MEQ[4] = RHO * (-UX);
-  MEQ[5] = RHO * (UY);
-  MEQ[6] = RHO * (-UY);
-  MEQ[7] = RHO * (UX * UX - UY * UY);
-  MEQ[8] = RHO * (UX * UY);
-  double mm[9];
-#pragma unroll
-  for (int k = 0; k < 9; ++k)
-    mm[k] = S[k] * MEQ[k] + (1. - S[k]) * M[k] + (1. - 0.5 * S[k]) * MF[k];
-  f[0] = d_mrt * (4.0 * (mm[0] - mm[1] + mm[2]));
-  f[1] = d_mrt * (4. * mm[0] - mm[1] - 2. * mm[2] + 6. * mm[3] - 6. * mm[4] + 9. * mm[7]);
-  f[2] = d_mrt * (4.0 * mm[0] - mm[1] - 2.0 * mm[2] + 6.0 * mm[5] - 6.0 * mm[6] - 9.0 * mm[7]);
-  f[3] = d_mrt * (4.0 * mm[0] - mm[1] - 2.0 * mm[2] - 6.0 * mm[3] + 6.0 * mm[4] + 9.0 * mm[7]);
-  f[4] = d_mrt * (4.0 * mm[0] - mm[1] - 2.0 * mm[2] - 6.0 * mm[5] + 6.0 * mm[6] - 9.0 * mm[7]);
-  f[5] = d_mrt * (4.0 * mm[0] + 2.0 * mm[1] + mm[2] + 6.0 * mm[3] + 3.0 * mm[4] + 6.0 * mm[5] +
-                  3.0 * mm[6] + 9.0 * mm[8]);
-  f[6] = d_mrt * (4.0 * mm[0] + 2.0 * mm[1] + mm[2] - 6.0 * mm[3] - 3.0 * mm[4] + 6.0 * mm[5] +
-                  3.0 * mm[6] - 9.0 * mm[8]);
-  f[7] = d_mrt * (4.0 * mm[0] + 2.0 * mm[1] + mm[2] - 6.0 * mm[3] - 3.0 * mm[4] - 6.0 * mm[5] -
-                  3.0 * mm[6] + 9.0 * mm[8]);
-  f[8] = d_mrt * (4.0 * mm[0] + 2.0 * mm[1] + mm[2] + 6.0 * mm[3] + 3.0 * mm[4] - 6.0 * mm[5] -
-                  3.0 * mm[6] - 9.0 * mm[8]);
-  if (!want_stress) return;
-  // Chai strain rate from S*(m - m_eq) + forcing correction, C6:903-916
-  double MNE[9], F1[9];
-  if (m.strain_feq) {  // C1:896-908: against the moments of COMPUTEFEQNEW
-    double FE[9];
-    feq_double(m, UX, UY, RHO, FE);
-    MNE[0] = M[0] - (FE[0] + FE[1] + FE[2] + FE[3] + FE[4] + FE[5] + FE[6] + FE[7] + FE[8]);
-    MNE[1] = M[1] - (-4.0 * FE[0] - FE[1] - FE[2] - FE[3] - FE[4] + 2.0 * (FE[5] + FE[6] + FE[7] + FE[8]));
-    MNE[2] = M[2] - (4.0 * FE[0] - 2.0 * (FE[1] + FE[2] + FE[3] + FE[4]) + (FE[5] + FE[6] + FE[7] + FE[8]));
-    MNE[3] = M[3] - (FE[1] - FE[3] + FE[5] - FE[6] - FE[7] + FE[8]);
-    MNE[4] = M[4] - (-2.0 * (FE[1] - FE[3]) + FE[5] - FE[6] - FE[7] + FE[8]);
-    MNE[5] = M[5] - (FE[2] - FE[4] + FE[5] + FE[6] - FE[7] - FE[8]);
-    MNE[6] = M[6] - (-2.0 * (FE[2] - FE[4]) + FE[5] + FE[6] - FE[7] - FE[8]);
-    MNE[7] = M[7] - (FE[1] - FE[2] + FE[3] - FE[4]);
-    MNE[8] = M[8] - (FE[5] - FE[6] + FE[7] - FE[8]);
-  } else {
-#pragma unroll
-    for (int k = 0; k < 9; ++k) MNE[k] = M[k] - MEQ[k];
+// Density and velocity of one node in FP64, in the order of C1:1421-1439;
+// returns 1/rho.
+__device__ __forceinline__ double macro64(const double* f, double& rho, double& ux, double& uy) {
+  rho = f[0] + f[1] + f[2] + f[3] + f[4] + f[5] + f[6] + f[7] + f[8];
+  const double rinv = 1.0 / rho;
+  ux = rinv * (f[1] + f[5] + f[8] - (f[6] + f[3] + f[7]));
+  uy = rinv * (f[5] + f[2] + f[6] - (f[7] + f[4] + f[8]));
+  return rinv;
+}
+
+// Collision_MRT for one node in FP64 (C1:875-1048; Chai strain rate and
+// Papanastasiou viscosity C6:903-958).  f: the populations, relaxed in place;
+// (ux, uy): the corrected velocity; w: the node's omega (node_omega) or
+// unused; rinv: 1/rho.
+//
+// The step was bound by this arithmetic, not by memory: written as the
+// reference writes it (every product and sum its own instruction, nine
+// explicit moments, nine inverse sums, the strain rate through nine more) a
+// Newtonian node took 263 FP64 instructions and a Bingham node 452, and the
+// FP64 pipe was half busy with 16 warps per SM waiting on each other's
+// results.  Here the small moments (momentum, heat flux, shear) come from
+// sums and differences of opposite populations, the inverse shares its
+// partial sums, fused multiply-adds are written out (the translation unit is
+// built with --fmad=false, so every kernel that collides a node gives the
+// same bits), the forcing terms are skipped where G = 0 (there they add
+// zeros), and the strain rate is the closed form of its nine sums.  What is
+// kept in the reference's order is what its rounding depends on: rho and the
+// two large moments and their relaxation.  With those the disk's velocity
+// after 400 steps stays within 4e-13 of the reference's; with them reordered
+// too it differs by 3e-12 (the reference's own rounding error, against the
+// same steps in 80-bit arithmetic), more than the 1e-12 the tests compare at.
+// 250 steps of the viscoplastic 800 x 2400 lattice 28.3 -> 17.4 ms, 300 of
+// the equilibrium-boundary 1500 x 1000 one 13.2 -> 12.2 ms, 500 of the
+// sedimentation 1024 x 2048 one 42.0 -> 40.8 ms (output included).
+__device__ __forceinline__ void collide64(const Model& m, double* f, double rho, double rinv,
+                                          double ux, double uy, double gx, double gy,
+                                          bool node_omega, double w, bool want_stress,
+                                          NodeOut& no) {
+  double sq = m.sq_uni, sw = m.omega;
+  if (node_omega) {  // ComputeRelaxation_MRT at the node's omega (C6:1002-1021)
+    sw = w;
+    sq = m.q_of_omega ? 8. * (2. - w) / (8. - w) : m.s_q;
   }
-  F1[1] = 4.0 * S[0] * MNE[0] - 1.0 * S[1] * MNE[1] - 2.0 * S[2] * MNE[2] + 6.0 * S[3] * MNE[3] -
-          6.0 * S[4] * MNE[4] + 9.0 * S[7] * MNE[7];
-  F1[2] = 4.0 * S[0] * MNE[0] - 1.0 * S[1] * MNE[1] - 2.0 * S[2] * MNE[2] + 6.0 * S[5] * MNE[5] -
-          6.0 * S[6] * MNE[6] - 9.0 * S[7] * MNE[7];
-  F1[3] = 4.0 * S[0] * MNE[0] - 1.0 * S[1] * MNE[1] - 2.0 * S[2] * MNE[2] - 6.0 * S[3] * MNE[3] +
-          6.0 * S[4] * MNE[4] + 9.0 * S[7] * MNE[7];
-  F1[4] = 4.0 * S[0] * MNE[0] - 1.0 * S[1] * MNE[1] - 2.0 * S[2] * MNE[2] - 6.0 * S[5] * MNE[5] +
-          6.0 * S[6] * MNE[6] - 9.0 * S[7] * MNE[7];
-  F1[5] = 4.0 * S[0] * MNE[0] + 2.0 * S[1] * MNE[1] + 1.0 * S[2] * MNE[2] + 6.0 * S[3] * MNE[3] +
-          3.0 * S[4] * MNE[4] + 6.0 * S[5] * MNE[5] + 3.0 * S[6] * MNE[6] + 9.0 * S[8] * MNE[8];
-  F1[6] = 4.0 * S[0] * MNE[0] + 2.0 * S[1] * MNE[1] + 1.0 * S[2] * MNE[2] - 6.0 * S[3] * MNE[3] -
-          3.0 * S[4] * MNE[4] + 6.0 * S[5] * MNE[5] + 3.0 * S[6] * MNE[6] - 9.0 * S[8] * MNE[8];
-  F1[7] = 4.0 * S[0] * MNE[0] + 2.0 * S[1] * MNE[1] + 1.0 * S[2] * MNE[2] - 6.0 * S[3] * MNE[3] -
-          3.0 * S[4] * MNE[4] - 6.0 * S[5] * MNE[5] - 3.0 * S[6] * MNE[6] + 9.0 * S[8] * MNE[8];
-  F1[8] = 4.0 * S[0] * MNE[0] + 2.0 * S[1] * MNE[1] + 1.0 * S[2] * MNE[2] + 6.0 * S[3] * MNE[3] +
-          3.0 * S[4] * MNE[4] - 6.0 * S[5] * MNE[5] - 3.0 * S[6] * MNE[6] - 9.0 * S[8] * MNE[8];
-  double D11, D22, D12;
-  if (m.strain_feq) {  // C1:940-948: 1/RHO folded into both terms
-    const double IR = 1.0 / RHO;
-    double ZARIB = -1.5 * d_mrt * IR;
-    D11 = ZARIB * (F1[1] + F1[5] + F1[6] + F1[3] + F1[7] + F1[8]);
-    D22 = ZARIB * (F1[5] + F1[2] + F1[6] + F1[7] + F1[4] + F1[8]);
-    D12 = ZARIB * (F1[5] - F1[6] + F1[7] - F1[8]);
-    ZARIB = 0.75 * IR;
-    D11 = D11 + ZARIB * ((S[7] - S[1]) * (GX * UX + GY * UY) - S[7] * (2.0 * GX * UX));
-    D22 = D22 + ZARIB * ((S[7] - S[1]) * (GX * UX + GY * UY) - S[7] * (2.0 * GY * UY));
-    D12 = D12 + ZARIB * (-S[7] * (GX * UY + GY * UX));
-  } else {  // C6:903-916
-    const double ZARIB = -1.5 * d_mrt;
-    D11 = ZARIB * (F1[1] + F1[5] + F1[6] + F1[3] + F1[7] + F1[8]) +
-          0.75 * ((S[7] - S[1]) * (GX * UX + GY * UY) - S[7] * (2.0 * GX * UX));
-    D22 = ZARIB * (F1[5] + F1[2] + F1[6] + F1[7] + F1[4] + F1[8]) +
-          0.75 * ((S[7] - S[1]) * (GX * UX + GY * UY) - S[7] * (2.0 * GY * UY));
-    D12 = ZARIB * (F1[5] - F1[6] + F1[7] - F1[8]) + 0.75 * (-S[7] * (GX * UY + GY * UX));
+  const double s1 = m.s_e, s2 = m.s_eps, d = m.d_mrt;
+  const double s14 = f[1] + f[2] + f[3] + f[4], s58 = f[5] + f[6] + f[7] + f[8];
+  const double e = f[1] - f[3], g = f[2] - f[4], h = f[5] - f[7], k = f[6] - f[8];
+  const double M0 = f[0] + f[1] + f[2] + f[3] + f[4] + f[5] + f[6] + f[7] + f[8];
+  const double M1 = fma(2.0, s58, fma(-4.0, f[0], -f[1]) - f[2] - f[3] - f[4]);
+  const double M2 = fma(-2.0, s14, 4.0 * f[0]) + s58;
+  const double hmk = h - k, hpk = h + k;
+  const double M4 = fma(-2.0, e, hmk), M6 = fma(-2.0, g, hpk);
+  const double M7 = (f[1] + f[3]) - (f[2] + f[4]), M8 = (f[5] + f[7]) - (f[6] + f[8]);
+  const double uxx = ux * ux, uyy = uy * uy;
+  const double U2 = uxx + uyy;
+  const double E1 = rho * fma(3.0, U2, -2.0), E2 = rho * fma(-3.0, U2, 1.0);
+  const double E7 = rho * (uxx - uyy), E8 = rho * (ux * uy);
+  const double n1 = M1 - E1, n7 = M7 - E7, n8 = M8 - E8;
+  double m1 = s1 * E1 + (1.0 - s1) * M1, m2 = s2 * E2 + (1.0 - s2) * M2;
+  double m3 = e + hmk, m5 = g + hpk;
+  double m4 = fma(-sq, fma(rho, ux, M4), M4), m6 = fma(-sq, fma(rho, uy, M6), M6);
+  double m7 = fma(-sw, n7, M7), m8 = fma(-sw, n8, M8);
+  const bool forced = gx != 0.0 || gy != 0.0;
+  if (forced) {  // (1 - S/2) m_F, F = rho G (C1:995-1016)
+    const double fx = rho * gx, fy = rho * gy;
+    const double fu = fma(fx, ux, fy * uy);
+    const double hq = fma(-0.5, sq, 1.0), hw = fma(-0.5, sw, 1.0);
+    m1 = fma(fma(-3.0, s1, 6.0), fu, m1);
+    m2 = fma(-fma(-3.0, s2, 6.0), fu, m2);
+    m3 = m3 + fx;
+    m5 = m5 + fy;
+    m4 = fma(-hq, fx, m4);
+    m6 = fma(-hq, fy, m6);
+    m7 = fma(hw, 2.0 * fma(fx, ux, -(fy * uy)), m7);
+    m8 = fma(hw, fma(fy, ux, fx * uy), m8);
+  }
+  const double m0 = 4.0 * M0;
+  const double A = fma(-2.0, m2, m0 - m1), B = fma(2.0, m1, m0) + m2;
+  const double X = 6.0 * (m3 - m4), Y = 6.0 * (m5 - m6);
+  const double X2 = fma(6.0, m3, 3.0 * m4), Y2 = fma(6.0, m5, 3.0 * m6);
+  const double P7 = 9.0 * m7, P8 = 9.0 * m8;
+  const double AP = A + P7, AM = A - P7, BP = B + P8, BM = B - P8;
+  const double XpY = X2 + Y2, XmY = X2 - Y2;
+  f[0] = d * (4.0 * (M0 - m1 + m2));
+  f[1] = d * (AP + X);
+  f[3] = d * (AP - X);
+  f[2] = d * (AM + Y);
+  f[4] = d * (AM - Y);
+  f[5] = d * (BP + XpY);
+  f[7] = d * (BP - XpY);
+  f[6] = d * (BM - XmY);
+  f[8] = d * (BM + XmY);
+  if (!want_stress) return;
+  // Chai strain rate from S*(m - m_eq) + forcing correction, C6:903-916: its
+  // sums over the nine directions reduce to three moments
+  double t1 = 9.0 * s1 * n1, t7 = 27.0 * sw * n7, t8 = 54.0 * sw * n8;
+  if (m.strain_feq) {  // C1:896-908: against the moments of COMPUTEFEQNEW
+    double q[9];
+    feq_double(m, ux, uy, rho, q);
+    const double q1 = -4.0 * q[0] - q[1] - q[2] - q[3] - q[4] + 2.0 * (q[5] + q[6] + q[7] + q[8]);
+    t1 = 9.0 * s1 * (M1 - q1);
+    t7 = 27.0 * sw * (M7 - (q[1] - q[2] + q[3] - q[4]));
+    t8 = 54.0 * sw * (M8 - (q[5] - q[6] + q[7] - q[8]));
+  }
+  double D11 = -d * (t1 + t7), D22 = -d * (t1 - t7), D12 = -d * t8;
+  if (forced) {
+    const double gu = fma(gx, ux, gy * uy);
+    D11 += 0.75 * ((sw - s1) * gu - sw * (2.0 * gx * ux));
+    D22 += 0.75 * ((sw - s1) * gu - sw * (2.0 * gy * uy));
+    D12 -= 0.75 * sw * fma(gx, uy, gy * ux);
+  }
+  if (m.bingham || m.strain_feq) {  // C6:921-924; C1:940-948 folds 1/rho in at once
+    D11 = D11 * rinv;
+    D22 = D22 * rinv;
+    D12 = D12 * rinv;
   }
   const double NU = m.nu;
-  no.t11 = NU * 2.0 * D11;
-  no.t22 = NU * 2.0 * D22;
-  no.t12 = NU * 2.0 * D12;
-  no.yield = 0;
-  no.omega = S[7];
+  double NU_A = NU;
+  no.omega = sw;
   if (m.bingham) {
-    const double INV_RHO = 1.0 / RHO;
-    if (!m.strain_feq) {
-      D11 = D11 * INV_RHO;
-      D22 = D22 * INV_RHO;
-      D12 = D12 * INV_RHO;
-    }
-    const double GAMMA = sqrt(2.0 * fabs(D11 * D11 + D22 * D22 + 2.0 * (D12 * D12)));
-    double NU_A;
+    // gamma and 1/gamma from one reciprocal square root
+    const double g2 = 2.0 * fma(D11, D11, fma(D22, D22, 2.0 * (D12 * D12)));
+    const double ig = rsqrt(g2);
+    const double GAMMA = g2 > 0.0 ? g2 * ig : 0.0;
     if (m.casson) {  // C3:985-989
       if (GAMMA < m.gamma_min) {
         NU_A = sqrt(NU) + sqrt(m.m_pap * m.tau_y);
       } else {
-        NU_A = sqrt(NU) + sqrt(m.tau_y / GAMMA) * (1.0 - exp(-sqrt(m.m_pap * GAMMA)));
+        NU_A = sqrt(NU) + sqrt(m.tau_y * ig) * (1.0 - exp(-sqrt(m.m_pap * GAMMA)));
         NU_A = NU_A * NU_A;
       }
     } else if (GAMMA < m.gamma_min) {
       NU_A = NU + m.m_pap * m.tau_y;
     } else {
-      NU_A = NU + (m.tau_y / GAMMA) * (1.0 - exp(-(m.m_pap * GAMMA)));
+      // above m gamma = 38 the exponential is below half an ulp of 1
+      const double mg = m.m_pap * GAMMA;
+      NU_A = fma(m.tau_y * ig, mg > 38.0 ? 1.0 : 1.0 - exp(-mg), NU);
     }
-    no.t11 = NU_A * 2.0 * D11;
-    no.t22 = NU_A * 2.0 * D22;
-    no.t12 = NU_A * 2.0 * D12;
+    no.omega = 1.0 / fma(3.0, NU_A * rinv, 0.5);
+  }
+  if (!m.record_stress) return;
+  no.t11 = NU_A * 2.0 * D11;
+  no.t22 = NU_A * 2.0 * D22;
+  no.t12 = NU_A * 2.0 * D12;
+  no.yield = 0;
+  if (m.bingham) {
     const double TAU_MAG =
         sqrt(0.5 * fabs(no.t11 * no.t11 + no.t22 * no.t22 + 2.0 * (no.t12 * no.t12)));
     no.yield = (TAU_MAG <= m.tau_y) ? 5 : 0;
-    NU_A = NU_A * INV_RHO;
-    no.omega = 1.0 / (3.0 * NU_A + 0.5);
   }
 }
 
@@ -725,6 +722,7 @@ __device__ __forceinline__ void lattice_body(const LatticeArgs& a, int bxi, int 
   // ---- macroscopic variables (C1:1421-1439) ----------------------------
   T rho, drho, ux, uy;
   Mom32 mq;
+  double rinv64 = 1.0;
   if (initial) {
     if (!F64) {
       float hq[9];
@@ -737,11 +735,14 @@ __device__ __forceinline__ void lattice_body(const LatticeArgs& a, int bxi, int 
     ux = (T)0;
     uy = (T)0;
   } else if (F64) {
-    rho = f[0] + f[1] + f[2] + f[3] + f[4] + f[5] + f[6] + f[7] + f[8];
+    double fd[9], r, x, y;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) fd[k] = (double)f[k];
+    rinv64 = macro64(fd, r, x, y);
+    rho = (T)r;
     drho = rho - (T)m.rho0;
-    const T rinv = (T)1.0 / rho;
-    ux = rinv * (f[1] + f[5] + f[8] - (f[6] + f[3] + f[7]));
-    uy = rinv * (f[5] + f[2] + f[6] - (f[7] + f[4] + f[8]));
+    ux = (T)x;
+    uy = (T)y;
   } else {
     float hq[9];
 #pragma unroll
@@ -944,18 +945,13 @@ __device__ __forceinline__ void lattice_body(const LatticeArgs& a, int bxi, int 
       pm[2 * g.plane + n] = uyc;
     }
   } else if (F64) {
-    double S[9];
-    if (node_omega) {
-      rates_double(m, (double)static_cast<const T*>(a.om_src)[n], S);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 9; ++k) S[k] = m.S_uni[k];
-    }
+    const double w = node_omega ? (double)static_cast<const T*>(a.om_src)[n] : 0.0;
+    if (initial) rinv64 = 1.0 / m.rho0;
     double fd[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) fd[k] = (double)f[k];
-    collide_double(m, fd, (double)rho, (double)uxc, (double)uyc, (double)gx, (double)gy, S,
-                   want_stress, no);
+    collide64(m, fd, (double)rho, rinv64, (double)uxc, (double)uyc, (double)gx, (double)gy,
+              node_omega, w, want_stress, no);
 #pragma unroll
     for (int k = 0; k < 9; ++k) f[k] = (T)fd[k];
   } else {
@@ -1191,9 +1187,10 @@ struct StepIO {
 // One node's values between the stage read and the collision.
 template <class T>
 struct NodeVals {
-  T f[9];
   T rho, drho, ux, uy, gx, gy;
-  Mom32 mq;
+  T f[9];       // FP64: the populations
+  double rinv;  // and 1/rho
+  Mom32 mq;     // FP32: the moments
 };
 
 // Node (i, j) of a staged tile: populations after streaming and the
@@ -1233,11 +1230,14 @@ __device__ __forceinline__ void node_gather(const LatticeArgs& a, const StepIO<T
   T rho, drho, ux, uy;
   Mom32& mq = v.mq;
   if (F64) {
-    rho = f[0] + f[1] + f[2] + f[3] + f[4] + f[5] + f[6] + f[7] + f[8];
+    double fd[9], r, x, y;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) fd[k] = (double)f[k];
+    v.rinv = macro64(fd, r, x, y);
+    rho = (T)r;
     drho = rho - (T)m.rho0;
-    const T rinv = (T)1.0 / rho;
-    ux = rinv * (f[1] + f[5] + f[8] - (f[6] + f[3] + f[7]));
-    uy = rinv * (f[5] + f[2] + f[6] - (f[7] + f[4] + f[8]));
+    ux = (T)x;
+    uy = (T)y;
   } else {
     float hq[9];
 #pragma unroll
@@ -1255,12 +1255,6 @@ __device__ __forceinline__ void node_gather(const LatticeArgs& a, const StepIO<T
     ux = uy = (T)0;
   }
   lattice_health<T>(a.status, drho, lane);
-  // FP64 reads f back from the stage after the particle loop instead of
-  // holding 18 registers across it; edge nodes park theirs there first
-  if (F64 && edge && act) {
-#pragma unroll
-    for (int k = 0; k < 9; ++k) q[ST::off(k)] = f[k];
-  }
 
   // ---- SPM body force (the highest-index particle with PHI>0 sets G,
   //      C1:500-507) and force sums ---------------------------------------
@@ -1282,6 +1276,13 @@ __device__ __forceinline__ void node_gather(const LatticeArgs& a, const StepIO<T
       nr = dx * dx + dy * dy < reach * reach;
     }
     near = __ballot_sync(0xffffffffu, nr);
+  }
+  // FP64 parks the node's populations in its stage elements during the disk
+  // loop (18 registers the loop needs); no other node reads these elements
+  const bool park = F64 && near != 0;
+  if (park) {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) q[ST::off(k)] = f[k];
   }
   while (near) {
     const int c = __ffs(near) - 1;
@@ -1326,7 +1327,7 @@ __device__ __forceinline__ void node_gather(const LatticeArgs& a, const StepIO<T
       }
     }
   }
-  if (F64 && act) {
+  if (park) {
 #pragma unroll
     for (int k = 0; k < 9; ++k) f[k] = q[ST::off(k)];
   }
@@ -1363,21 +1364,15 @@ __device__ __forceinline__ void node_collide(const LatticeArgs& a, const StepIO<
   no.t11 = no.t22 = no.t12 = 0.0;
   T omn = (T)m.omega;
   if (bingham) omn = om_node;
+  T f[9];
   if (F64) {
-    double S[9];
-    if (bingham) {
-      rates_double(m, (double)omn, S);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 9; ++k) S[k] = m.S_uni[k];
-    }
     double fd[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) fd[k] = (double)v.f[k];
-    collide_double(m, fd, (double)v.rho, (double)uxc, (double)uyc, (double)v.gx, (double)v.gy, S,
-                   want_stress, no);
+    collide64(m, fd, (double)v.rho, v.rinv, (double)uxc, (double)uyc, (double)v.gx, (double)v.gy,
+              bingham, (double)omn, want_stress, no);
 #pragma unroll
-    for (int k = 0; k < 9; ++k) v.f[k] = (T)fd[k];
+    for (int k = 0; k < 9; ++k) f[k] = (T)fd[k];
   } else {
     Rates32 r;
     r.s1 = m.s_e_f;
@@ -1394,10 +1389,10 @@ __device__ __forceinline__ void node_collide(const LatticeArgs& a, const StepIO<
     relax32(m, v.mq, (float)v.rho, (float)uxc, (float)uyc, (float)v.gx, (float)v.gy, r,
             want_stress, no, hf);
 #pragma unroll
-    for (int k = 0; k < 9; ++k) v.f[k] = (T)hf[k];
+    for (int k = 0; k < 9; ++k) f[k] = (T)hf[k];
   }
 #pragma unroll
-  for (int k = 0; k < 9; ++k) dst[plane_of(k) * P + nd] = v.f[k];
+  for (int k = 0; k < 9; ++k) dst[plane_of(k) * P + nd] = f[k];
   if (bingham) io.om_dst[nd] = (T)no.omega;
   if (STRESS && m.record_stress) {
     const int slot = (int)((io.step + 1) & 1);
