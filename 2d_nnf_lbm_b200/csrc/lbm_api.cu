@@ -47,8 +47,12 @@ struct lbm_sim {
   int np = 0;
   int np_cap = 0;
   double* ps = nullptr;                // [PS][npad]
+  double* ps_alt = nullptr;            // the other copy (k_steps ping-pongs them)
   int npad = 32;
-  unsigned long long* facc = nullptr;  // [6][npad] FORCE accumulators
+  unsigned long long* facc = nullptr;  // [6][npad] FORCE accumulators in use, one of
+  unsigned long long* facc3 = nullptr;  // [3][6][npad] (k_steps rotates them)
+  bool lists_stale = false;  // k_steps moved the disks: the tile and pair lists are old
+  unsigned* steps_bar = nullptr;       // k_steps' grid barrier
   int* rec_slot = nullptr;
   int* tile_count = nullptr;
   int* tile_list = nullptr;
@@ -69,7 +73,8 @@ struct lbm_sim {
   // scalars
   unsigned long long* mass_acc = nullptr;
   long long* d_kk = nullptr;
-  double* stale_dpw = nullptr;
+  double* stale_dpw = nullptr;   // D_PW in use, one of
+  double* stale_dpw2 = nullptr;  // [2] (k_steps alternates them)
   int* h_status = nullptr;  // pinned copy of d_status, refreshed after each call
   int* d_status = nullptr;  // sticky ST_* bits written by the kernels
   // history
@@ -136,6 +141,12 @@ struct lbm_sim {
 namespace {
 
 constexpr int NOUT = 7;  // ux uy rho phi gx gy pnode
+constexpr int STEPS_MAX_LAUNCH = 1024;  // time steps per launch of k_steps
+#ifndef LBM_STEPS_MAX_NODES
+#define LBM_STEPS_MAX_NODES 400000
+#endif
+constexpr long long STEPS_MAX_NODES = LBM_STEPS_MAX_NODES;
+constexpr long long STEPS_NODES_PER_DISK = 700;
 
 int cuda_fail(cudaError_t e) {
   if (e == cudaErrorMemoryAllocation) return LBM_E_NOMEM;
@@ -421,9 +432,15 @@ int ring_wait(lbm_sim* h, long long r) {
   return LBM_E_STATE;
 }
 
+int launch_tiles(lbm_sim* h);
+
 // Fields of step kk in h->out (and F after BC in h->out_f when want_f).
 int compute_output(lbm_sim* h, bool want_f) {
   if (h->out_kk == h->kk && (!want_f || h->out_f)) return LBM_OK;
+  if (h->lists_stale) {
+    int rc = launch_tiles(h);
+    if (rc) return rc;
+  }
   LatticeArgs a = lattice_args(h);
   a.src = h->f[h->cur ^ 1];
   a.om_src = h->om[h->cur ^ 1];
@@ -448,8 +465,9 @@ int setup_particle_buffers(lbm_sim* h, int np, double dmax) {
   const bool keep_s = h->series && h->p.series_every > 0 && series_len == h->series_len &&
                       series_cap == h->series_cap;
   if (!keep_p) {
-    dfree(h->ps); dfree(h->facc); dfree(h->nbr); dfree(h->nbr_count); dfree(h->nbr_xy);
-    h->ps = nullptr; h->facc = nullptr; h->nbr = nullptr; h->nbr_count = nullptr;
+    dfree(h->ps); dfree(h->ps_alt); dfree(h->facc3);
+    dfree(h->nbr); dfree(h->nbr_count); dfree(h->nbr_xy);
+    h->ps = h->ps_alt = nullptr; h->facc = h->facc3 = nullptr; h->nbr = nullptr; h->nbr_count = nullptr;
     h->nbr_xy = nullptr;
   }
   // records of the old disk set (its record length) are dropped
@@ -475,13 +493,15 @@ int setup_particle_buffers(lbm_sim* h, int np, double dmax) {
   const size_t npa = (size_t)h->npad;
   if (!keep_p) {
     if ((rc = dalloc(&h->ps, npa * PS))) return rc;
-    if ((rc = dalloc(&h->facc, npa * 6))) return rc;
+    if ((rc = dalloc(&h->ps_alt, npa * PS))) return rc;
+    if ((rc = dalloc(&h->facc3, npa * 18))) return rc;
+    h->facc = h->facc3;
     if ((rc = dalloc(&h->nbr, npa * MAX_NEIGH))) return rc;
     if ((rc = dalloc(&h->nbr_count, npa))) return rc;
     if ((rc = dalloc(&h->nbr_xy, npa * 2))) return rc;
   }
   CK(cudaMemsetAsync(h->ps, 0, sizeof(double) * npa * PS, h->stream));
-  CK(cudaMemsetAsync(h->facc, 0, sizeof(unsigned long long) * npa * 6, h->stream));
+  CK(cudaMemsetAsync(h->facc3, 0, sizeof(unsigned long long) * npa * 18, h->stream));
   CK(cudaMemsetAsync(h->nbr_count, 0, sizeof(int) * npa, h->stream));
   CK(cudaMemsetAsync(h->nbr_xy, 0, sizeof(double) * npa * 2, h->stream));
   CK(cudaMemsetAsync(h->tile_count, 0, sizeof(int) * 2 * h->g.ltx * h->g.lty, h->stream));
@@ -529,6 +549,7 @@ int launch_tiles(lbm_sim* h) {
   CK(launch_tiles_only(pa, h->stream));
   CK(launch_tile_order(pa, 0, h->stream));
   CK(launch_tile_order(pa, 1, h->stream));
+  h->lists_stale = false;
   return LBM_OK;
 }
 
@@ -746,12 +767,13 @@ void destroy_buffers(lbm_sim* h) {
   }
   dfree(h->rec);
   dfree(h->ring);
-  dfree(h->ps); dfree(h->facc); dfree(h->nbr); dfree(h->nbr_count); dfree(h->nbr_xy);
+  dfree(h->ps); dfree(h->ps_alt); dfree(h->facc3); dfree(h->steps_bar);
+  dfree(h->nbr); dfree(h->nbr_count); dfree(h->nbr_xy);
   dfree(h->tile_count); dfree(h->tile_list); dfree(h->tile_cur); dfree(h->pair_rebuild);
   dfree(h->tile_order); dfree(h->n_unlisted); dfree(h->work_ctr);
   dfree(h->rec_slot);
   dfree(h->mass_acc);
-  dfree(h->d_kk); dfree(h->stale_dpw);
+  dfree(h->d_kk); dfree(h->stale_dpw2);
   dfree(h->series); dfree(h->out); dfree(h->out_f); dfree(h->d_status);
   dfree(h->u0); dfree(h->err_part);
   if (h->series_pin) cudaFreeHost(h->series_pin);
@@ -819,6 +841,10 @@ int enqueue_step(lbm_sim* h) {
     int rc = ring_wait(h, (h->kk + 1) / every - 1);
     if (rc) return rc;
   }
+  if (h->lists_stale) {
+    int rc = launch_tiles(h);
+    if (rc) return rc;
+  }
   if (h->prof) {
     if (h->ev_used + 3 > 3 * 65536) {
       int rc = profile_flush(h);
@@ -836,6 +862,67 @@ int enqueue_step(lbm_sim* h) {
   h->cur ^= 1;
   h->prev_post_bc = false;
   h->partials_valid = true;
+  return LBM_OK;
+}
+
+// Whether the handle steps several steps per launch (k_steps).  The line is
+// where the two ways take the same time (us per step, k_steps / the particle
+// and step kernels): FP64 201 x 601 7.7 / 11.2, 401 x 801 11.3 / 13.5, 501 x
+// 1001 16.2 / 15.7; FP32 6.8 / 10.6, 9.7 / 10.5, 12.4 / 11.9.  A step of k_steps grows faster with
+// the lattice (its blocks load by node, the step kernel by TMA tiles) and
+// with the disks (each block updates all of them): at 513 x 513 with 20 disks
+// 12.2 / 12.8 (FP64), with 200 disks 18.8 / 18.5.
+bool steps_resident(const lbm_sim* h) {
+  return !h->prof && !h->m.bgk && h->np <= STEPS_MAX_DISKS &&
+         nodes(h) + STEPS_NODES_PER_DISK * h->np <= STEPS_MAX_NODES;
+}
+
+// Up to `left` time steps in one launch on the handle's stream; *done: how
+// many (bounded by the room in the history ring).
+int enqueue_steps(lbm_sim* h, int left, int* done) {
+  const int every = h->p.series_every;
+  int n = std::min(left, STEPS_MAX_LAUNCH);
+  if (h->series && every > 0) {
+    if ((h->kk + 1) / every - h->copied_kk / every > h->series_cap) {
+      int rc = series_enqueue(h);  // the ring slots are copied before reuse
+      if (rc) return rc;
+    }
+    const long long last = (h->copied_kk / every + h->series_cap + 1) * (long long)every - 1;
+    n = (int)std::min<long long>(n, last - h->kk);
+    if ((h->kk + n) / every > h->kk / every) {
+      int rc = ring_wait(h, (h->kk + n) / every - 1);
+      if (rc) return rc;
+    }
+  }
+  StepsArgs q{};
+  for (int b = 0; b < 2; ++b) {
+    q.f[b] = h->f[h->cur ^ b];
+    q.om[b] = h->om[h->cur ^ b];
+  }
+  q.ps[0] = h->ps;
+  q.ps[1] = h->ps_alt;
+  q.facc = h->facc3;
+  q.facc0 = (int)((h->facc - h->facc3) / (6 * (ptrdiff_t)h->npad));
+  q.stale = h->stale_dpw2;
+  q.stale0 = (int)(h->stale_dpw - h->stale_dpw2);
+  q.bar = h->steps_bar;
+  q.kk0 = h->kk;
+  q.nsteps = n;
+  q.decode0 = h->partials_valid ? 1 : 0;
+  const LatticeArgs a = lattice_args(h);
+  const ParticleArgs pa = particle_args(h);
+  CK(cudaMemsetAsync(h->steps_bar, 0, sizeof(unsigned), h->stream));
+  CK(h->prec == LBM_FP64 ? launch_steps_fp64(a, pa, q, h->stream)
+                         : launch_steps_fp32(a, pa, q, h->stream));
+  h->kk += n;
+  h->cur ^= n & 1;
+  std::swap(h->ps, h->ps_alt);
+  h->stale_dpw = h->stale_dpw2 + (q.stale0 ^ 1);
+  h->facc = h->facc3 + (size_t)((q.facc0 + n) % 3) * 6 * h->npad;
+  h->prev_post_bc = false;
+  h->partials_valid = true;
+  h->lists_stale = true;
+  *done = n;
   return LBM_OK;
 }
 
@@ -1074,7 +1161,9 @@ int lbm_create(const lbm_params* pin, lbm_sim** out) {
   cudaMemsetAsync(h->tile_cur, 0, 2 * sizeof(int), h->stream);
   cudaMemsetAsync(h->pair_rebuild, 0, sizeof(int), h->stream);
   if ((rc = dalloc(&h->d_kk, 1))) return fail(rc);
-  if ((rc = dalloc(&h->stale_dpw, 1))) return fail(rc);
+  if ((rc = dalloc(&h->stale_dpw2, 2))) return fail(rc);
+  h->stale_dpw = h->stale_dpw2;
+  if ((rc = dalloc(&h->steps_bar, 1))) return fail(rc);
   if ((rc = dalloc(&h->out, (size_t)NOUT * nodes(h)))) return fail(rc);
   cudaMemsetAsync(h->f[0], 0, fbytes, h->stream);
   cudaMemsetAsync(h->f[1], 0, fbytes, h->stream);
@@ -1147,9 +1236,11 @@ int lbm_step(lbm_sim* h, int32_t nsteps) {
   int st = sticky_status(h);
   if (st) return st;
   cudaSetDevice(h->p.device);
-  for (int32_t s = 0; s < nsteps; ++s) {
-    int rc = enqueue_step(h);
+  for (int32_t s = 0; s < nsteps;) {
+    int n = 1;
+    int rc = steps_resident(h) ? enqueue_steps(h, nsteps - s, &n) : enqueue_step(h);
     if (rc) return rc;
+    s += n;
   }
   if (h->series) {
     int rc = series_enqueue(h);  // this call's records, copied behind its kernels
@@ -2126,6 +2217,7 @@ int lbm_batch_step(lbm_batch* b, int32_t nsteps) {
   for (lbm_sim* h : b->sims) {
     int st = sticky_status(h);
     if (st) return st;
+    if (h->lists_stale && (st = launch_tiles(h))) return st;
     CK(cudaStreamSynchronize(h->stream));  // the handles' own work first
   }
   int rc;

@@ -1,6 +1,7 @@
 // lbm_fp32.cu -- FP32 shifted-population instantiation of the lattice kernel
 // (h = f - w_k*rho0 stored and computed in FP32; reductions in FP64).
 #include "lbm_lattice.cuh"
+#include "lbm_steps.cuh"
 
 namespace lbm {
 cudaError_t launch_init_fp32(const LatticeArgs& a, cudaStream_t s) {
@@ -46,5 +47,9 @@ cudaError_t batch_tma_prepare_fp32(int stress, int* blocks_per_sm) {
 }
 cudaError_t launch_bgk_step_fp32(const LatticeArgs& a, cudaStream_t s) {
   return launch_mode<float>(a, s, MODE_STEP);
+}
+cudaError_t launch_steps_fp32(const LatticeArgs& a, const ParticleArgs& p, const StepsArgs& q,
+                              cudaStream_t s) {
+  return launch_steps<float>(a, p, q, s);
 }
 }  // namespace lbm

@@ -3,6 +3,7 @@
 // reference's order, so the only differences from the FP64 oracle come from
 // sin() and from the order of the force reductions.
 #include "lbm_lattice.cuh"
+#include "lbm_steps.cuh"
 
 namespace lbm {
 cudaError_t launch_init_fp64(const LatticeArgs& a, cudaStream_t s) {
@@ -31,5 +32,9 @@ cudaError_t batch_tma_prepare_fp64(int stress, int* blocks_per_sm) {
 }
 cudaError_t launch_bgk_step_fp64(const LatticeArgs& a, cudaStream_t s) {
   return launch_mode<double>(a, s, MODE_STEP);
+}
+cudaError_t launch_steps_fp64(const LatticeArgs& a, const ParticleArgs& p, const StepsArgs& q,
+                              cudaStream_t s) {
+  return launch_steps<double>(a, p, q, s);
 }
 }  // namespace lbm

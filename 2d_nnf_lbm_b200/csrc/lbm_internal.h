@@ -211,6 +211,26 @@ struct LatticeArgs {
   int initial;           // 1: state is INITIALIZE (rho0, u=0, G=0)
 };
 
+// Several time steps of a small simulation in one launch (lbm_steps.cuh).
+constexpr int STEPS_MAX_DISKS = 256;
+struct StepsArgs {
+  void* f[2];                // step s (1..nsteps) reads f[(s-1)&1], writes f[s&1]
+  void* om[2];
+  double* ps[2];             // [PS][npad] disk state: read, and written at the end
+  unsigned long long* facc;  // [3][6][npad]: step s adds to (facc0 + s) % 3
+  int facc0;
+  double* stale;             // [2]: D_PW, read at stale0, written at stale0 ^ 1
+  int stale0;
+  unsigned* bar;             // grid barrier, zero at the start
+  long long kk0;             // steps done before the launch
+  int nsteps;
+  int decode0;               // the accumulators hold FORCE of step kk0
+};
+cudaError_t launch_steps_fp64(const LatticeArgs& a, const ParticleArgs& p, const StepsArgs& q,
+                              cudaStream_t s);
+cudaError_t launch_steps_fp32(const LatticeArgs& a, const ParticleArgs& p, const StepsArgs& q,
+                              cudaStream_t s);
+
 // Launchers (defined in lbm_fp64.cu / lbm_fp32.cu).
 cudaError_t launch_init_fp64(const LatticeArgs& a, cudaStream_t s);
 cudaError_t launch_step_fp64(const LatticeArgs& a, const CUtensorMap* tm, const CUtensorMap* tmo,

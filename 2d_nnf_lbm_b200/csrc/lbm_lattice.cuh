@@ -39,6 +39,14 @@ __device__ __forceinline__ double wexact(int k) {
   return k == 0 ? 4.0 / 9.0 : (k < 5 ? 1.0 / 9.0 : 1.0 / 36.0);
 }
 
+// A load of data that other blocks write during the launch (CG: past the L1
+// cache), or an ordinary one.
+template <bool CG, class T>
+__device__ __forceinline__ T ld(const T* p) {
+  if constexpr (CG) return __ldcg(p);
+  else return *p;
+}
+
 // ---------------------------------------------------------------------------
 // COMPUTEFEQNEW (C1:1157-1175) in double.
 __device__ __forceinline__ void feq_double(const Model& m, double ux, double uy, double rho,
@@ -92,22 +100,25 @@ __device__ __forceinline__ void ring_store(const LatticeArgs& a, int i, int j, i
 // bracket of COMPUTEFEQNEW, so no O(1) terms cancel.
 __device__ __forceinline__ void feq_shift32(const Model& m, float dr, float x, float y, float* h) {
   const float r0 = m.rho0_f;
-  const float U2 = x * x + y * y;
+  const float xx = x * x, yy = y * y, xy9 = 9.f * x * y;
+  const float U2 = 3.f * (xx + yy);
+  const float X = fmaf(9.f, xx, -U2), Y = fmaf(9.f, yy, -U2);
+  const float P = U2 + xy9, M = U2 - xy9;
   float d[9];  // B_k - B_k(0)
-  d[0] = -3.f * U2;
-  d[1] = 6.f * x + 9.f * x * x - 3.f * U2;
-  d[2] = 6.f * y + 9.f * y * y - 3.f * U2;
-  d[3] = -6.f * x + 9.f * x * x - 3.f * U2;
-  d[4] = -6.f * y + 9.f * y * y - 3.f * U2;
-  d[5] = 3.f * (x + y) + 9.f * x * y + 3.f * U2;
-  d[6] = -3.f * (x - y) - 9.f * x * y + 3.f * U2;
-  d[7] = -3.f * (x + y) + 9.f * x * y + 3.f * U2;
-  d[8] = 3.f * (x - y) - 9.f * x * y + 3.f * U2;
+  d[0] = -U2;
+  d[1] = fmaf(6.f, x, X);
+  d[2] = fmaf(6.f, y, Y);
+  d[3] = fmaf(-6.f, x, X);
+  d[4] = fmaf(-6.f, y, Y);
+  d[5] = fmaf(3.f, x + y, P);
+  d[6] = fmaf(-3.f, x - y, M);
+  d[7] = fmaf(-3.f, x + y, P);
+  d[8] = fmaf(3.f, x - y, M);
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
     const float W = m.w_init_f[k == 0 ? 0 : (k < 5 ? 1 : 2)];
     const float B = (k == 0 || k < 5 ? 2.f : 1.f) + d[k];
-    h[k] = W * (dr * B + r0 * d[k]) + m.eq_c_f[k];
+    h[k] = fmaf(W, fmaf(dr, B, r0 * d[k]), m.eq_c_f[k]);
   }
 }
 
@@ -131,12 +142,12 @@ __device__ __forceinline__ void bgk_source(const T* W, T rho, T ux, T uy, T gx, 
 // arithmetic.  FP32 (shifted populations, the ring holding rho - rho0):
 // h_k = W_k (drho B_k + rho0 (B_k - B_k(0))) + rho0 (W_k B_k(0) - w_k), with
 // B_k the bracket of COMPUTEFEQNEW, so no O(1) terms cancel.
-template <class T>
+template <class T, bool CG = false>
 __device__ __forceinline__ void edge_equilibrium(const LatticeArgs& a, int i, int j, int par,
                                                  T* f) {
   const int s = ring_edge_slot(a.g, i, j), n = a.ring_n;
   const T* q = static_cast<const T*>(a.ring) + (long long)par * 3 * n;
-  const T r = q[s], ux = q[n + s], uy = q[2 * n + s];
+  const T r = ld<CG>(q + s), ux = ld<CG>(q + n + s), uy = ld<CG>(q + 2 * n + s);
   if (sizeof(T) == 8) {
     double fe[9];
     feq_double(a.m, (double)ux, (double)uy, (double)r, fe);
@@ -166,12 +177,12 @@ __device__ __forceinline__ double phi_double(double di, double dj, double R, dou
 }
 
 __device__ __forceinline__ float phi_float(float di, float dj, float R, float zeta, float pi) {
-  const float D = R - sqrtf(di * di + dj * dj);
+  const float D = R - sqrtf(fmaf(di, di, dj * dj));
   float phi = 0.0f;
   if (D <= -0.5f * zeta)
     phi = 0.0f;
   else if (fabsf(D) < 0.5f * zeta)
-    phi = 0.5f * (__sinf(pi * D / zeta) + 1.0f);  // |argument| < pi/2
+    phi = fmaf(0.5f, __sinf(pi * D / zeta), 0.5f);  // |argument| < pi/2
   else if (D >= 0.5f * zeta)
     phi = 1.0f;
   return phi;
@@ -360,8 +371,8 @@ __device__ __forceinline__ Mom32 moments32(const float* h) {
   q.drho = h[0] + (ab + cd);
   q.jx = e + hmk;
   q.jy = g + hpk;
-  q.m1 = fmaf(2.0f, cd, -ab) - 4.0f * h[0];
-  q.m2 = fmaf(4.0f, h[0], cd) - 2.0f * ab;
+  q.m1 = fmaf(-4.0f, h[0], fmaf(2.0f, cd, -ab));
+  q.m2 = fmaf(-2.0f, ab, fmaf(4.0f, h[0], cd));
   q.m4 = fmaf(-2.0f, e, hmk);
   q.m6 = fmaf(-2.0f, g, hpk);
   q.m7 = a - b;
@@ -374,29 +385,53 @@ __device__ __forceinline__ Mom32 moments32(const float* h) {
 __device__ __forceinline__ void relax32(const Model& m, const Mom32& q, float rho, float ux,
                                         float uy, float gx, float gy, const Rates32& r,
                                         bool want_stress, NodeOut& no, float* h) {
-  const float FX = rho * gx, FY = rho * gy;
   const float uxx = ux * ux, uyy = uy * uy;
   const float ru2 = 3.0f * rho * (uxx + uyy);
   const float e1 = fmaf(-2.0f, q.drho, ru2);
   const float e2 = q.drho - ru2;
-  const float e4 = -rho * ux;
-  const float e6 = -rho * uy;
-  const float e7 = rho * (uxx - uyy);
-  const float e8 = rho * (ux * uy);
-  const float fu = fmaf(FX, ux, FY * uy);
-  const float cw = 1.0f - 0.5f * r.sw, cq = 1.0f - 0.5f * r.sq;
-  const float p0 = q.drho;
-  const float p1 = fmaf(r.s1, e1 - q.m1, q.m1) + (6.0f - 3.0f * r.s1) * fu;
-  const float p2 = fmaf(r.s2, e2 - q.m2, q.m2) - (6.0f - 3.0f * r.s2) * fu;
-  const float p3 = q.jx + FX;
-  const float p5 = q.jy + FY;
-  const float p4 = fmaf(r.sq, e4 - q.m4, q.m4) - cq * FX;
-  const float p6 = fmaf(r.sq, e6 - q.m6, q.m6) - cq * FY;
-  const float p7 = fmaf(r.sw, e7 - q.m7, q.m7) + cw * (2.0f * fmaf(FX, ux, -FY * uy));
-  const float p8 = fmaf(r.sw, e8 - q.m8, q.m8) + cw * fmaf(FY, ux, FX * uy);
+  const float n1 = q.m1 - e1;
+  const float n7 = fmaf(-rho, uxx - uyy, q.m7);
+  const float n8 = fmaf(-rho, ux * uy, q.m8);
   const float d = m.d_mrt_f;
-  const float A = fmaf(4.0f, p0, -p1) - 2.0f * p2;
-  const float B = fmaf(4.0f, p0, 2.0f * p1) + p2;
+  const bool forced = gx != 0.0f || gy != 0.0f;
+  // closed form of the Chai strain rate (C6:903-916) with S0 = S3 = S5 = 0
+  float D11 = 0.0f, D22 = 0.0f, D12 = 0.0f;
+  if (want_stress) {
+    const float t1 = 9.0f * r.s1 * n1, t7 = 27.0f * r.sw * n7;
+    D11 = -d * (t1 + t7);
+    D22 = -d * (t1 - t7);
+    D12 = -54.0f * d * r.sw * n8;
+  }
+  if (want_stress && forced) {
+    const float gu = fmaf(gx, ux, gy * uy);
+    const float tg = (r.sw - r.s1) * gu;
+    D11 = fmaf(0.75f, fmaf(-r.sw, 2.0f * gx * ux, tg), D11);
+    D22 = fmaf(0.75f, fmaf(-r.sw, 2.0f * gy * uy, tg), D22);
+    D12 = fmaf(-0.75f, r.sw * fmaf(gx, uy, gy * ux), D12);
+  }
+  const float p0 = q.drho;
+  float p1 = fmaf(-r.s1, n1, q.m1);
+  float p2 = fmaf(r.s2, e2 - q.m2, q.m2);
+  float p3 = q.jx, p5 = q.jy;
+  float p4 = fmaf(-r.sq, fmaf(rho, ux, q.m4), q.m4);
+  float p6 = fmaf(-r.sq, fmaf(rho, uy, q.m6), q.m6);
+  float p7 = fmaf(-r.sw, n7, q.m7);
+  float p8 = fmaf(-r.sw, n8, q.m8);
+  if (__builtin_expect(forced, 0)) {  // (1 - S/2) m_F, F = rho G: zeros elsewhere
+    const float FX = rho * gx, FY = rho * gy;
+    const float fu = fmaf(FX, ux, FY * uy);
+    const float cw = fmaf(-0.5f, r.sw, 1.0f), cq = fmaf(-0.5f, r.sq, 1.0f);
+    p1 = fmaf(fmaf(-3.0f, r.s1, 6.0f), fu, p1);
+    p2 = fmaf(-fmaf(-3.0f, r.s2, 6.0f), fu, p2);
+    p3 += FX;
+    p5 += FY;
+    p4 = fmaf(-cq, FX, p4);
+    p6 = fmaf(-cq, FY, p6);
+    p7 = fmaf(cw, 2.0f * fmaf(FX, ux, -FY * uy), p7);
+    p8 = fmaf(cw, fmaf(FY, ux, FX * uy), p8);
+  }
+  const float A = fmaf(-2.0f, p2, fmaf(4.0f, p0, -p1));
+  const float B = fmaf(4.0f, p0, fmaf(2.0f, p1, p2));
   const float X = 6.0f * (p3 - p4), Y = 6.0f * (p5 - p6);
   const float X2 = fmaf(6.0f, p3, 3.0f * p4), Y2 = fmaf(6.0f, p5, 3.0f * p6);
   const float P7 = 9.0f * p7, P8 = 9.0f * p8;
@@ -412,13 +447,6 @@ __device__ __forceinline__ void relax32(const Model& m, const Mom32& q, float rh
   h[6] = fmaf(d, BM - XmY, m.shift_f[6]);
   h[8] = fmaf(d, BM + XmY, m.shift_f[8]);
   if (!want_stress) return;
-  // closed form of the Chai strain rate (C6:903-916) with S0 = S3 = S5 = 0
-  const float n1 = q.m1 - e1, n7 = q.m7 - e7, n8 = q.m8 - e8;
-  const float t1 = 9.0f * r.s1 * n1, t7 = 27.0f * r.sw * n7;
-  const float gu = gx * ux + gy * uy;
-  float D11 = -d * (t1 + t7) + 0.75f * ((r.sw - r.s1) * gu - r.sw * (2.0f * gx * ux));
-  float D22 = -d * (t1 - t7) + 0.75f * ((r.sw - r.s1) * gu - r.sw * (2.0f * gy * uy));
-  float D12 = -54.0f * d * r.sw * n8 + 0.75f * (-r.sw * (gx * uy + gy * ux));
   if (m.strain_feq) {  // C1:940-948 divides both terms by rho (FP32: the
     // moments of COMPUTEFEQNEW equal the moment-space equilibrium here)
     const float ir = 1.0f / rho;
@@ -443,7 +471,7 @@ __device__ __forceinline__ void relax32(const Model& m, const Mom32& q, float rh
       D22 *= inv_rho;
       D12 *= inv_rho;
     }
-    const float g2 = 2.0f * fabsf(D11 * D11 + D22 * D22 + 2.0f * (D12 * D12));
+    const float g2 = 2.0f * fmaf(D11, D11, fmaf(D22, D22, 2.0f * (D12 * D12)));
     const float gam = g2 > 0.0f ? g2 * rsqrtf(g2) : 0.0f;
     const float ty = m.tau_y_f;
     float nua;
@@ -461,7 +489,7 @@ __device__ __forceinline__ void relax32(const Model& m, const Mom32& q, float rh
       // above m gamma = 18 it rounds to exactly 1 in FP32 (e^-18 < 2^-25),
       // so yielded fluid skips the exponential
       const float mg = m.m_pap_f * gam;
-      nua = NU + __fdividef(ty, gam) * (mg > 18.0f ? 1.0f : -expm1f(-mg));
+      nua = fmaf(__fdividef(ty, gam), mg > 18.0f ? 1.0f : -expm1f(-mg), NU);
     }
     const float t11 = nua * 2.0f * D11, t22 = nua * 2.0f * D22, t12 = nua * 2.0f * D12;
     no.t11 = t11;
@@ -471,7 +499,7 @@ __device__ __forceinline__ void relax32(const Model& m, const Mom32& q, float rh
       const float tm = sqrtf(0.5f * fabsf(t11 * t11 + t22 * t22 + 2.0f * (t12 * t12)));
       no.yield = (tm <= ty) ? 5 : 0;
     }
-    no.omega = __fdividef(1.0f, 3.0f * (nua * inv_rho) + 0.5f);
+    no.omega = __fdividef(1.0f, fmaf(3.0f, nua * inv_rho, 0.5f));
   }
 }
 
@@ -480,7 +508,7 @@ __device__ __forceinline__ void relax32(const Model& m, const Mom32& q, float rh
 // lattice keep the node's own post-collision value (C1:1195-1199); the
 // boundary routine then overwrites the unknowns.  Wall velocities are zero
 // in every reference case, which reduces the moving-wall terms to +-0.
-template <class T>
+template <class T, bool CG = false>
 __device__ __forceinline__ void pull_bc(const T* __restrict__ src, const Geometry& g, int bc,
                                         int i, int j, T* f) {
   const long long P = g.plane;
@@ -488,18 +516,19 @@ __device__ __forceinline__ void pull_bc(const T* __restrict__ src, const Geometr
   const int pt = g.pitch;
   const bool L = (i == 0), R = (i == g.nx), B = (j == 0), U = (j == g.ny);
   const T* s0 = src + n;
-  f[0] = s0[0];
-  f[1] = !L ? s0[plane_of(1) * P - 1] : s0[plane_of(1) * P];
-  f[2] = !B ? s0[plane_of(2) * P - pt] : s0[plane_of(2) * P];
-  f[3] = !R ? s0[plane_of(3) * P + 1] : s0[plane_of(3) * P];
-  f[4] = !U ? s0[plane_of(4) * P + pt] : s0[plane_of(4) * P];
-  f[5] = (!L && !B) ? s0[plane_of(5) * P - pt - 1] : s0[plane_of(5) * P];
-  f[6] = (!R && !B) ? s0[plane_of(6) * P - pt + 1] : s0[plane_of(6) * P];
-  f[7] = (!R && !U) ? s0[plane_of(7) * P + pt + 1] : s0[plane_of(7) * P];
-  f[8] = (!L && !U) ? s0[plane_of(8) * P + pt - 1] : s0[plane_of(8) * P];
+  // (one load each: the address is selected, not the value)
+  f[0] = ld<CG>(s0);
+  f[1] = ld<CG>(s0 + (plane_of(1) * P - (L ? 0 : 1)));
+  f[2] = ld<CG>(s0 + (plane_of(2) * P - (B ? 0 : pt)));
+  f[3] = ld<CG>(s0 + (plane_of(3) * P + (R ? 0 : 1)));
+  f[4] = ld<CG>(s0 + (plane_of(4) * P + (U ? 0 : pt)));
+  f[5] = ld<CG>(s0 + (plane_of(5) * P - (L || B ? 0 : pt + 1)));
+  f[6] = ld<CG>(s0 + (plane_of(6) * P - (R || B ? 0 : pt - 1)));
+  f[7] = ld<CG>(s0 + (plane_of(7) * P + (R || U ? 0 : pt + 1)));
+  f[8] = ld<CG>(s0 + (plane_of(8) * P + (L || U ? 0 : pt - 1)));
   if (!(L || R || B || U)) return;
   // own post-collision populations F_POST(k,i,j)
-#define FPOST(k) src[plane_of(k) * P + n]
+#define FPOST(k) ld<CG>(src + plane_of(k) * P + n)
   if ((L || R) && (B || U)) {
     // corners: half-way bounce-back of 3 of the 5 unknowns (C1:1390-1414)
     if (L && B) { f[1] = FPOST(3); f[5] = FPOST(7); f[2] = FPOST(4); }
@@ -535,21 +564,21 @@ __device__ __forceinline__ void pull_bc(const T* __restrict__ src, const Geometr
 #undef FPOST
 }
 
-template <class T>
+template <class T, bool CG = false>
 __device__ __forceinline__ void pull_interior(const T* __restrict__ src, const Geometry& g,
                                               long long n, T* f) {
   const long long P = g.plane;
   const int pt = g.pitch;
   const T* s0 = src + n;
-  f[0] = s0[0];
-  f[1] = s0[plane_of(1) * P - 1];
-  f[2] = s0[plane_of(2) * P - pt];
-  f[3] = s0[plane_of(3) * P + 1];
-  f[4] = s0[plane_of(4) * P + pt];
-  f[5] = s0[plane_of(5) * P - pt - 1];
-  f[6] = s0[plane_of(6) * P - pt + 1];
-  f[7] = s0[plane_of(7) * P + pt + 1];
-  f[8] = s0[plane_of(8) * P + pt - 1];
+  f[0] = ld<CG>(s0);
+  f[1] = ld<CG>(s0 + plane_of(1) * P - 1);
+  f[2] = ld<CG>(s0 + plane_of(2) * P - pt);
+  f[3] = ld<CG>(s0 + plane_of(3) * P + 1);
+  f[4] = ld<CG>(s0 + plane_of(4) * P + pt);
+  f[5] = ld<CG>(s0 + plane_of(5) * P - pt - 1);
+  f[6] = ld<CG>(s0 + plane_of(6) * P - pt + 1);
+  f[7] = ld<CG>(s0 + plane_of(7) * P + pt + 1);
+  f[8] = ld<CG>(s0 + plane_of(8) * P + pt - 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -1054,6 +1083,16 @@ struct TileCand {
   void* dst;
   const void* om_src;
   void* om_dst;
+  // what node_force reads
+  static constexpr int CAP = MAX_TILE_CAND;
+  __device__ __forceinline__ double x(int c) const { return px[c]; }
+  __device__ __forceinline__ double y(int c) const { return py[c]; }
+  __device__ __forceinline__ double diam(int c) const { return pd[c]; }
+  __device__ __forceinline__ double u(int c) const { return pu[c]; }
+  __device__ __forceinline__ double v(int c) const { return pv[c]; }
+  __device__ __forceinline__ double w(int c) const { return pw[c]; }
+  __device__ __forceinline__ int id(int c) const { return idx[c]; }
+  __device__ __forceinline__ unsigned long long* facc(const LatticeArgs& a) const { return a.facc; }
 };
 
 template <class T, class ST = Stage<T>>
@@ -1193,39 +1232,41 @@ struct NodeVals {
   Mom32 mq;     // FP32: the moments
 };
 
-// Node (i, j) of a staged tile: populations after streaming and the
-// boundary conditions, macroscopic variables, lattice health, SPM body force
-// (the highest-index disk with PHI > 0 sets G) and the warp's force sums.
-// Every lane of the warp calls it (act: the node is in the lattice; edge:
-// it gathers its populations from global memory); q points at the node's
-// stage elements.  PDL: the force accumulators are touched only after
-// griddepcontrol.wait (the particle kernel that zeroes them may still run).
-template <class T, bool PDL, class ST = Stage<T>>
-__device__ __forceinline__ void node_gather(const LatticeArgs& a, const StepIO<T>& io,
-                                            const TileCand& C, T* const q, int i, int j,
-                                            bool act, bool edge, int lane, bool& waited,
-                                            NodeVals<T>& v) {
-  constexpr bool F64 = sizeof(T) == 8;
-  const Geometry& g = a.g;
-  const Model& m = a.m;
-  const T* __restrict__ src = io.src;
-  // ---- streaming + boundary conditions --------------------------------
-  // Nodes inside the lattice take the streamed values from the stage;
-  // nodes on its edge gather theirs with the boundary conditions.
-  T* const f = v.f;
+// Node (i, j) of a staged tile: the populations after streaming and the
+// boundary conditions.  Nodes inside the lattice take the streamed values
+// from the stage (q: the node's stage elements), nodes on its edge (edge)
+// gather theirs from global memory.
+template <class T, class ST>
+__device__ __forceinline__ void node_stream(const LatticeArgs& a, const StepIO<T>& io, const T* q,
+                                            int i, int j, bool act, bool edge, T* f) {
   if (!edge) {
 #pragma unroll
     for (int k = 0; k < 9; ++k) f[k] = q[ST::off(k)];
   } else if (act) {
-    if (m.bc == BC_EQUILIBRIUM)
+    if (a.m.bc == BC_EQUILIBRIUM)
       edge_equilibrium<T>(a, i, j, (int)((io.step - 1) & 1), f);
     else
-      pull_bc<T>(src, g, m.bc, i, j, f);
+      pull_bc<T>(io.src, a.g, a.m.bc, i, j, f);
   } else {
 #pragma unroll
     for (int k = 0; k < 9; ++k) f[k] = (T)0;
   }
+}
 
+// Node (i, j) from its populations v.f: macroscopic variables, lattice
+// health, SPM body force (the highest-index disk with PHI > 0 sets G) and the
+// warp's force sums.  Every lane of the warp calls it (act: the
+// node is in the lattice; the warp's nodes are 32 neighbours of row j).  PDL:
+// the force accumulators are touched only after griddepcontrol.wait (the
+// particle kernel that zeroes them may still run).  q: the node's stage
+// elements, where FP64 parks its populations (ST void: none).
+template <class T, bool PDL, class ST, class Cand>
+__device__ __forceinline__ void node_force(const LatticeArgs& a, const Cand& C,
+                                           T* const q, int i, int j, bool act, int lane,
+                                           bool& waited, NodeVals<T>& v) {
+  constexpr bool F64 = sizeof(T) == 8;
+  const Model& m = a.m;
+  T* const f = v.f;
   // ---- macroscopic variables (C1:1421-1439) ---------------------------
   T rho, drho, ux, uy;
   Mom32& mq = v.mq;
@@ -1265,71 +1306,91 @@ __device__ __forceinline__ void node_gather(const LatticeArgs& a, const StepIO<T
   // R + zeta/2 + 1e-3 from the centre, so PHI is 0 there in either
   // precision (rounding of the node distance is far below 1e-3) and the
   // skipped iterations would add nothing.
-  unsigned near = 0;
-  {
-    bool nr = false;
-    if (lane < C.n) {  // the warp's nodes: columns i - lane .. i - lane + 31
-      const double dl = (double)(i - lane) - C.px[lane], dr = dl + 31.0;
-      const double dx = dl > 0.0 ? dl : (dr < 0.0 ? -dr : 0.0);
-      const double dy = (double)j - C.py[lane];
-      const double reach = 0.5 * C.pd[lane] + 0.5 * m.zeta + 1e-3;
-      nr = dx * dx + dy * dy < reach * reach;
+  bool parked = false;
+  auto chunk = [&](int c0) {  // candidates c0 .. c0 + 31
+    unsigned near = 0;
+    {
+      bool nr = false;
+      const int c = c0 + lane;
+      if (c < C.n) {  // the warp's nodes: columns i - lane .. i - lane + 31
+        const double dl = (double)(i - lane) - C.x(c), dr = dl + 31.0;
+        const double dx = dl > 0.0 ? dl : (dr < 0.0 ? -dr : 0.0);
+        const double dy = (double)j - C.y(c);
+        const double reach = 0.5 * C.diam(c) + 0.5 * m.zeta + 1e-3;
+        nr = dx * dx + dy * dy < reach * reach;
+      }
+      near = __ballot_sync(0xffffffffu, nr);
     }
-    near = __ballot_sync(0xffffffffu, nr);
-  }
-  // FP64 parks the node's populations in its stage elements during the disk
-  // loop (18 registers the loop needs); no other node reads these elements
-  const bool park = F64 && near != 0;
-  if (park) {
+    // FP64 parks the node's populations in its stage elements during the disk
+    // loop (18 registers the loop needs); no other node reads these elements
+    if constexpr (F64 && !std::is_void_v<ST>) {
+      if (near != 0) {
+        parked = true;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) q[ST::off(k)] = f[k];
-  }
-  while (near) {
-    const int c = __ffs(near) - 1;
-    near &= near - 1;
-    double fx = 0.0, fy = 0.0, tz = 0.0;
-    bool hit = false;
-    if (act) {
-      const double di = (double)i - C.px[c];
-      const double dj = (double)j - C.py[c];
-      T phi;
-      if (F64)
-        phi = (T)phi_double(di, dj, 0.5 * C.pd[c], m.zeta, m.pi);
-      else
-        phi = (T)phi_float((float)di, (float)dj, (float)(0.5 * C.pd[c]), m.zeta_f, m.pi_f);
-      if (phi > (T)0) {
-        hit = true;
-        const T uxp = (T)C.pu[c] - (T)C.pw[c] * (T)dj;
-        const T uyp = (T)C.pv[c] + (T)C.pw[c] * (T)di;
-        if (C.idx[c] > gbest) {
-          gbest = C.idx[c];
-          gx = phi * (uxp - ux);
-          gy = phi * (uyp - uy);
+        for (int k = 0; k < 9; ++k) q[ST::off(k)] = f[k];
+      }
+    }
+    while (near) {
+      const int c = c0 + __ffs(near) - 1;
+      near &= near - 1;
+      double fx = 0.0, fy = 0.0, tz = 0.0;
+      bool hit = false;
+      if (act) {
+        const double di = (double)i - C.x(c);
+        const double dj = (double)j - C.y(c);
+        T phi;
+        if (F64)
+          phi = (T)phi_double(di, dj, 0.5 * C.diam(c), m.zeta, m.pi);
+        else
+          phi = (T)phi_float((float)di, (float)dj, (float)(0.5 * C.diam(c)), m.zeta_f, m.pi_f);
+        if (phi > (T)0) {
+          hit = true;
+          T uxp, uyp;
+          if (F64) {
+            uxp = (T)C.u(c) - (T)C.w(c) * (T)dj;
+            uyp = (T)C.v(c) + (T)C.w(c) * (T)di;
+          } else {
+            uxp = fmaf(-(float)C.w(c), (float)dj, (float)C.u(c));
+            uyp = fmaf((float)C.w(c), (float)di, (float)C.v(c));
+          }
+          if (C.id(c) > gbest) {
+            gbest = C.id(c);
+            gx = phi * (uxp - ux);
+            gy = phi * (uyp - uy);
+          }
+          const T rp = rho * phi;
+          fx = (double)(rp * (ux - uxp));
+          fy = (double)(rp * (uy - uyp));
+          tz = (double)(rp * ((T)di * (uy - uyp) - (T)dj * (ux - uxp)));
         }
-        const T rp = rho * phi;
-        fx = (double)(rp * (ux - uxp));
-        fy = (double)(rp * (uy - uyp));
-        tz = (double)(rp * ((T)di * (uy - uyp) - (T)dj * (ux - uxp)));
+      }
+      if (__any_sync(0xffffffffu, hit)) {
+        // warp totals of (Fx, Fy, Tz) in lanes 0, 8, 16
+        const double tot = warp_sum3(fx, fy, tz, lane);
+        if (PDL && !waited) {  // the particle kernel has zeroed the accumulators
+          asm volatile("griddepcontrol.wait;" ::: "memory");
+          waited = true;
+        }
+        const int comp = lane >> 3;
+        if ((lane & 7) == 0 && comp < 3 && LBM_IN(C.id(c), a.np, a.status)) {
+          const long long st = a.npad;
+          unsigned long long* acc = C.facc(a) + C.id(c) + 2 * comp * st;
+          facc_add(acc, acc + st, tot);
+        }
       }
     }
-    if (__any_sync(0xffffffffu, hit)) {
-      // warp totals of (Fx, Fy, Tz) in lanes 0, 8, 16
-      const double tot = warp_sum3(fx, fy, tz, lane);
-      if (PDL && !waited) {  // the particle kernel has zeroed the accumulators
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        waited = true;
-      }
-      const int comp = lane >> 3;
-      if ((lane & 7) == 0 && comp < 3 && LBM_IN(C.idx[c], a.np, a.status)) {
-        const long long st = a.npad;
-        unsigned long long* acc = a.facc + C.idx[c] + 2 * comp * st;
-        facc_add(acc, acc + st, tot);
-      }
-    }
+  };
+  if constexpr (Cand::CAP <= 32) {
+    chunk(0);
+  } else {
+#pragma unroll 1
+    for (int c0 = 0; c0 < C.n; c0 += 32) chunk(c0);
   }
-  if (park) {
+  if constexpr (F64 && !std::is_void_v<ST>) {
+    if (parked) {
 #pragma unroll
-    for (int k = 0; k < 9; ++k) f[k] = q[ST::off(k)];
+      for (int k = 0; k < 9; ++k) f[k] = q[ST::off(k)];
+    }
   }
   v.rho = rho;
   v.drho = drho;
@@ -1642,7 +1703,8 @@ __device__ __forceinline__ void step_body(const LatticeArgs& a, const CUtensorMa
                              ? slot + ST::BYTES / (int)sizeof(T) + tid
                              : nullptr;
     NodeVals<T> v;
-    node_gather<T, true>(a, io, C, q, i, j, act, edge, lane, waited, v);
+    node_stream<T, ST>(a, io, q, i, j, act, edge, v.f);
+    node_force<T, true, ST>(a, C, q, i, j, act, lane, waited, v);
     // the node's omega, from the stage while it is still this tile's
     const T omn = (STRESS && m.bingham && act) ? (omq ? *omq : io.om_src[nd]) : (T)0;
     // the stage and its candidates are consumed
@@ -1736,7 +1798,7 @@ cudaError_t launch_step_tma(const LatticeArgs& a, const CUtensorMap* tm, const C
 // ring that the consumers read their model from.  A slot is rewritten only
 // after every consumer warp has finished the tile that used it (warps are at
 // most NSTAGE tiles apart, the ring holds 2 NSTAGE).  The node arithmetic is
-// k_step's (node_gather, node_collide).  Launches do not overlap: the
+// k_step's (node_stream, node_force, node_collide).  Launches do not overlap: the
 // batched particle kernel runs between two.
 constexpr int BATCH_ARGS_SLOTS = 2 * NSTAGE;
 
@@ -1959,7 +2021,8 @@ __global__ void __launch_bounds__(STEP_TPB, sizeof(T) == 8 ? 1 : LBM_STEP_MINB_F
                              ? slot + ST::BYTES / (int)sizeof(T) + tid
                              : nullptr;
     NodeVals<T> v;
-    node_gather<T, false, ST>(a, io, C, qp, i, j, act, edge, lane, waited, v);
+    node_stream<T, ST>(a, io, qp, i, j, act, edge, v.f);
+    node_force<T, false, ST>(a, C, qp, i, j, act, lane, waited, v);
     // the node's omega, from the stage while it is still this tile's
     const T omn = (STRESS && a.m.bingham && act) ? (omq ? *omq : io.om_src[nd]) : (T)0;
     // the stage and its candidates are consumed (the ring slot is not)

@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 #include <cstddef>
 
+#include "lbm_disk.cuh"
 #include "lbm_internal.h"
 
 namespace lbm {
@@ -46,31 +47,6 @@ static_assert(offsetof(PShared, x) >= (size_t)REC_STAGE * 12 * sizeof(double),
               "record staging fits in front of the centre arrays");
 
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
-
-// Pair force of (lo, hi), lo < hi, as the reference evaluates F_PP for
-// IP = lo, JP = hi (C3:758-766); the contact branch tests D_PP or the stale
-// wall distance D_PW.
-__device__ __forceinline__ void pair_force(const ParticleArgs& a, double ax, double ay, double ad,
-                                           double bx, double by, double bd, double test_stale,
-                                           double* F) {
-  const double ZITA = a.rep_zeta, CIJ = a.c_ij, EPS_P = a.eps_p, E_P = a.e_p;
-  const double dx = ax - bx, dy = ay - by;
-  const double D_PP = sqrt(dx * dx + dy * dy);
-  const double rsum = 0.5 * ad + 0.5 * bd;
-  const double test = a.contact == 1 ? test_stale : D_PP;
-  F[0] = 0.0;
-  F[1] = 0.0;
-  if (D_PP > rsum + ZITA) return;
-  const double q = (D_PP - 0.5 * ad - 0.5 * bd - ZITA) / ZITA;
-  if (D_PP <= rsum + ZITA && test > rsum) {
-    F[0] = EPS_P * CIJ * (q * q) * dx / D_PP;
-    F[1] = EPS_P * CIJ * (q * q) * dy / D_PP;
-  } else if (test <= rsum) {
-    const double e = E_P * CIJ * (rsum - D_PP) / ZITA;
-    F[0] = (EPS_P * CIJ * (q * q) + e) * dx / D_PP;
-    F[1] = (EPS_P * CIJ * (q * q) + e) * dy / D_PP;
-  }
-}
 
 // Insert disk p into the candidate lists of the tiles within R + zeta/2 + 1
 // + SKIN of (x, y); atomics are issued four at a time so latencies overlap.
@@ -353,10 +329,20 @@ __device__ __forceinline__ void particles_body(const ParticleArgs& a) {
   for (int p = tid; p < a.np; p += PBLK) {
     const PRef P{a.ps + p, a.npad};
     // issue every global load of this disk before the dependent arithmetic
-    const double u0 = P[P_U], u1 = P[P_V], u2 = P[P_W];
-    const double uo0 = P[P_UO], uo1 = P[P_VO], uo2 = P[P_WO];
-    const double frx = P[P_FX], fry = P[P_FY], frt = P[P_TZ];
-    const double rhop = P[P_RHO], M = P[P_M], I = P[P_I], ang = P[P_ANG];
+    DiskStep d;
+    d.u = P[P_U];
+    d.v = P[P_V];
+    d.w = P[P_W];
+    d.uo = P[P_UO];
+    d.vo = P[P_VO];
+    d.wo = P[P_WO];
+    d.fx = P[P_FX];
+    d.fy = P[P_FY];
+    d.tz = P[P_TZ];
+    d.rho_p = P[P_RHO];
+    d.M = P[P_M];
+    d.I = P[P_I];
+    d.ang = P[P_ANG];
     const double xt = P[P_XT], yt = P[P_YT];
     const double px = S.x[p], py = S.y[p], pd = S.d[p];
     // The neighbour count and the first 8 list entries load together (the
@@ -370,43 +356,11 @@ __device__ __forceinline__ void particles_body(const ParticleArgs& a) {
 #pragma unroll
       for (int k = 0; k < 8; ++k) nraw[k] = a.nbr[(long long)k * a.npad + p];
     }
-    double wf0[4] = {0.0, 0.0, 0.0, 0.0}, wf1[4] = {0.0, 0.0, 0.0, 0.0};
-    // walls (C1:735-768 mirror images; C3:775-804 wall disks)
+    double wf[4][2];
     if (a.wall_model != 2) {
-      const double ZITA = a.rep_zeta, CIJ = a.c_ij, EPS_W = a.eps_w, E_W = a.e_w;
-      const double x = px, y = py, D = pd;
       double D_PW = stale;
 #pragma unroll
-      for (int iw = 1; iw <= 4; ++iw) {
-        double rw0, rw1;
-        if (a.wall_model == 0) {
-          if (iw == 1) { rw0 = x; rw1 = -y; }
-          else if (iw == 2) { rw0 = 2.0 * (double)a.nx - x; rw1 = y; }
-          else if (iw == 3) { rw0 = x; rw1 = a.mirror_top - y; }
-          else { rw0 = a.mirror_left - x; rw1 = y; }
-        } else {
-          if (iw == 1) { rw0 = x; rw1 = -0.5 * D; }
-          else if (iw == 2) { rw0 = (double)a.nx + 0.5 * D; rw1 = y; }
-          else if (iw == 3) { rw0 = x; rw1 = (double)a.ny + 0.5 * D; }
-          else { rw0 = -0.5 * D; rw1 = y; }
-        }
-        const double ex = x - rw0, ey = y - rw1;
-        D_PW = sqrt(ex * ex + ey * ey);
-        double F0 = 0.0, F1 = 0.0;
-        if (!(D_PW > D + ZITA)) {
-          const double q = (D_PW - D - ZITA) / ZITA;
-          if (D_PW <= D + ZITA && D_PW > D) {
-            F0 = EPS_W * CIJ * (q * q) * ex / D_PW;
-            F1 = EPS_W * CIJ * (q * q) * ey / D_PW;
-          } else if (D_PW <= D) {
-            const double e = E_W * CIJ * (D - D_PW) / ZITA;
-            F0 = (EPS_W * CIJ * (q * q) + e) * ex / D_PW;
-            F1 = (EPS_W * CIJ * (q * q) + e) * ey / D_PW;
-          }
-        }
-        wf0[iw - 1] = F0;
-        wf1[iw - 1] = F1;
-      }
+      for (int iw = 1; iw <= 4; ++iw) D_PW = wall_force(a, iw, px, py, pd, wf[iw - 1]);
       if (p == a.np - 1) *a.stale_dpw = D_PW;
     }
     double fcx = 0.0, fcy = 0.0;
@@ -418,6 +372,9 @@ __device__ __forceinline__ void particles_body(const ParticleArgs& a) {
       for (int k = 0; k < nn; ++k) {
         const int q = k < 8 ? nbl[k] : a.nbr[(long long)k * a.npad + p];
         if (!LBM_IN(q, a.np, a.status)) continue;
+        // the lists reach SKIN beyond the range: most pairs end here, before
+        // the square root and the divisions
+        if (!pair_near(px, py, pd, S.x[q], S.y[q], S.d[q], a.rep_zeta)) continue;
         double F[2];
         if (q < p) {
           pair_force(a, S.x[q], S.y[q], S.d[q], px, py, pd, stale, F);
@@ -433,65 +390,46 @@ __device__ __forceinline__ void particles_body(const ParticleArgs& a) {
     if (a.wall_model != 2) {
 #pragma unroll
       for (int iw = 0; iw < 4; ++iw) {
-        fcx = fcx + wf0[iw];
-        fcy = fcy + wf1[iw];
+        fcx = fcx + wf[iw][0];
+        fcy = fcy + wf[iw][1];
       }
     }
+    d.x = px;
+    d.y = py;
+    d.fcx = fcx;
+    d.fcy = fcy;
+    newton_update(a, newton_terms(a, kk, d), d);
     P[P_FCX] = fcx;
     P[P_FCY] = fcy;
 
-    // Newton-Euler with internal-mass correction (C1:250-258, C6:312), or
-    // the prescribed oscillation (C4:222-228) with F_H_IN of this step's
-    // velocity change (C4:270-272)
-    const double RHO0 = a.rho0;
-    const double rr = RHO0 / rhop;
-    double fh0, fh1, fh2, v0, v1, v2;
-    if (a.motion == MOTION_OSCILLATE) {
-      v0 = -(a.osc_u * cos(((2.0 * a.pi) * (double)s_kk) / a.osc_period));
-      v1 = 0.0;
-      v2 = 0.0;
-      fh0 = rr * M * (v0 - u0);
-      fh1 = rr * M * (v1 - u1);
-      fh2 = rr * I * (v2 - u2);
-    } else {
-      fh0 = rr * M * (u0 - uo0);
-      fh1 = rr * M * (u1 - uo1);
-      fh2 = rr * I * (u2 - uo2);
-      v0 = u0 + frx / M + fh0 / M + fcx / M;
-      v1 = u1 + fry / M + fh1 / M + (1.0 - RHO0 / rhop) * a.gravity + fcy / M;
-      v2 = u2 + frt / I + fh2 / I;
-    }
-    const double nx_ = px + 0.5 * (v0 + u0);
-    const double ny_ = py + 0.5 * (v1 + u1);
-    P[P_FHX] = fh0;
-    P[P_FHY] = fh1;
-    P[P_FHT] = fh2;
-    P[P_UO] = u0;
-    P[P_VO] = u1;
-    P[P_WO] = u2;
-    P[P_U] = v0;
-    P[P_V] = v1;
-    P[P_W] = v2;
-    P[P_X] = nx_;
-    P[P_Y] = ny_;
-    const double nang = a.integrate_angle ? ang + 0.5 * (v2 + u2) : ang;
-    if (a.integrate_angle) P[P_ANG] = nang;
-    if (!isfinite(nx_) || !isfinite(ny_) || !isfinite(v0) || !isfinite(v1))
+    P[P_FHX] = d.fhx;
+    P[P_FHY] = d.fhy;
+    P[P_FHT] = d.fht;
+    P[P_UO] = d.uo;
+    P[P_VO] = d.vo;
+    P[P_WO] = d.wo;
+    P[P_U] = d.u;
+    P[P_V] = d.v;
+    P[P_W] = d.w;
+    P[P_X] = d.x;
+    P[P_Y] = d.y;
+    if (a.integrate_angle) P[P_ANG] = d.ang;
+    if (!isfinite(d.x) || !isfinite(d.y) || !isfinite(d.u) || !isfinite(d.v))
       atomicOr(a.status, ST_NAN);
-    else if (nx_ < 0.0 || nx_ > (double)a.nx || ny_ < 0.0 || ny_ > (double)a.ny)
+    else if (d.x < 0.0 || d.x > (double)a.nx || d.y < 0.0 || d.y > (double)a.ny)
       atomicOr(a.status, ST_PARTICLE);
     if (rec && p < a.series_np) {
       double* r = p < REC_STAGE ? rstage + 12LL * p : a.series + rslot * a.series_len + 2 + 12LL * p;
-      r[0] = nx_; r[1] = ny_; r[2] = nang;
-      r[3] = v0; r[4] = v1; r[5] = v2;
-      r[6] = frx; r[7] = fry; r[8] = frt;
-      r[9] = fh0; r[10] = fh1; r[11] = fh2;
+      r[0] = d.x; r[1] = d.y; r[2] = d.ang;
+      r[3] = d.u; r[4] = d.v; r[5] = d.w;
+      r[6] = d.fx; r[7] = d.fy; r[8] = d.tz;
+      r[9] = d.fhx; r[10] = d.fhy; r[11] = d.fht;
     }
     if (a.hist && kk < a.hist_n) {
       double* hr = a.hist + kk * (long long)PS * a.npad + p;
       for (int f = 0; f < PS; ++f) hr[(long long)f * a.npad] = P[f];
     }
-    const double tdx = nx_ - xt, tdy = ny_ - yt;
+    const double tdx = d.x - xt, tdy = d.y - yt;
     if (!(tdx * tdx + tdy * tdy <= 0.25 * SKIN * SKIN)) s_tiles = 1;
   }
   __syncthreads();
