@@ -26,6 +26,12 @@
 using namespace lbm;
 
 struct lbm_sim {
+  // device allocations that hold several of the buffers below (Block)
+  unsigned char* blk = nullptr;         // of the lattice (lbm_create)
+  unsigned char* blk_part = nullptr;    // of the disks
+  unsigned char* blk_series = nullptr;  // of the history
+  unsigned char* blk_adj = nullptr;     // of the adjoint: fields
+  unsigned char* blk_adj_np = nullptr;  // and per-disk state
   CUtensorMap tm[2];   // TMA descriptors of f[0], f[1] for the step kernel
   CUtensorMap tmo[2];  // and of om[0], om[1] (Bingham models; else copies of tm)
   lbm_params p;
@@ -53,6 +59,7 @@ struct lbm_sim {
   unsigned long long* facc3 = nullptr;  // [3][6][npad] (k_steps rotates them)
   bool lists_stale = false;  // k_steps moved the disks: the tile and pair lists are old
   unsigned* steps_bar = nullptr;       // k_steps' grid barrier
+  unsigned steps_bar_base = 0;         // its count so far
   int* rec_slot = nullptr;
   int* tile_count = nullptr;
   int* tile_list = nullptr;
@@ -65,7 +72,10 @@ struct lbm_sim {
   int* nbr_count = nullptr;
   double* nbr_xy = nullptr;
   int* pair_rebuild = nullptr;
-  double* ps_pin = nullptr;     // pinned staging of the particle upload [PS][npad]
+  // pinned staging of the particle upload [PS][npad] and of the particle read
+  // (records, then FORCE accumulators [6][npad]); for up to 32 disks the part
+  // of status_pin after the status word
+  double* ps_pin = nullptr;
   size_t ps_pin_n = 0;          // its size in doubles
   bool partials_valid = false;  // facc holds FORCE of the last lattice step
   int ncx = 1, ncy = 1;
@@ -75,6 +85,7 @@ struct lbm_sim {
   long long* d_kk = nullptr;
   double* stale_dpw = nullptr;   // D_PW in use, one of
   double* stale_dpw2 = nullptr;  // [2] (k_steps alternates them)
+  unsigned char* status_pin = nullptr;  // pinned: h_status, then ps_pin's first home
   int* h_status = nullptr;  // pinned copy of d_status, refreshed after each call
   int* d_status = nullptr;  // sticky ST_* bits written by the kernels
   // history
@@ -141,6 +152,7 @@ struct lbm_sim {
 namespace {
 
 constexpr int NOUT = 7;  // ux uy rho phi gx gy pnode
+constexpr size_t STATUS_PIN_HEAD = 64;  // bytes of status_pin before ps_pin
 constexpr int STEPS_MAX_LAUNCH = 1024;  // time steps per launch of k_steps
 #ifndef LBM_STEPS_MAX_NODES
 #define LBM_STEPS_MAX_NODES 400000
@@ -174,6 +186,31 @@ int dalloc(T** p, size_t count) {
 void dfree(void* p) {
   if (p) cudaFree(p);
 }
+
+// Several device buffers in one allocation (a cudaMalloc costs about 0.4 ms
+// and a cudaFree 0.35 ms however small the buffer; a handle had 25 of them).
+// add() notes a buffer, commit() allocates the block and sets the pointers;
+// the block, *base, is what is freed.
+struct Block {
+  struct Part {
+    void** p;
+    size_t off;
+  };
+  std::vector<Part> parts;
+  size_t size = 0;
+  template <class T>
+  void add(T** p, size_t count) {
+    *p = nullptr;
+    parts.push_back({reinterpret_cast<void**>(p), size});
+    size += (std::max<size_t>(count, 1) * sizeof(T) + 255) / 256 * 256;
+  }
+  int commit(unsigned char** base) {
+    int rc = dalloc(base, size);
+    if (rc) return rc;
+    for (const Part& q : parts) *q.p = *base + q.off;
+    return LBM_OK;
+  }
+};
 
 // All copies are ordered on the handle's (non-blocking) stream; copies to the
 // host wait for completion.
@@ -465,8 +502,8 @@ int setup_particle_buffers(lbm_sim* h, int np, double dmax) {
   const bool keep_s = h->series && h->p.series_every > 0 && series_len == h->series_len &&
                       series_cap == h->series_cap;
   if (!keep_p) {
-    dfree(h->ps); dfree(h->ps_alt); dfree(h->facc3);
-    dfree(h->nbr); dfree(h->nbr_count); dfree(h->nbr_xy);
+    dfree(h->blk_part);
+    h->blk_part = nullptr;
     h->ps = h->ps_alt = nullptr; h->facc = h->facc3 = nullptr; h->nbr = nullptr; h->nbr_count = nullptr;
     h->nbr_xy = nullptr;
   }
@@ -475,10 +512,10 @@ int setup_particle_buffers(lbm_sim* h, int np, double dmax) {
   h->host_series.clear();
   h->host_series_read = 0;
   if (!keep_s) {
-    dfree(h->series); dfree(h->mass_acc);
+    dfree(h->blk_series);
+    h->blk_series = nullptr;
     h->series = nullptr; h->mass_acc = nullptr;
-    if (h->series_pin) cudaFreeHost(h->series_pin);
-    if (h->mass_pin) cudaFreeHost(h->mass_pin);
+    if (h->series_pin) cudaFreeHost(h->series_pin);  // and mass_pin behind it
     h->series_pin = nullptr;
     h->mass_pin = nullptr;
   }
@@ -492,13 +529,15 @@ int setup_particle_buffers(lbm_sim* h, int np, double dmax) {
   h->npad = npad;
   const size_t npa = (size_t)h->npad;
   if (!keep_p) {
-    if ((rc = dalloc(&h->ps, npa * PS))) return rc;
-    if ((rc = dalloc(&h->ps_alt, npa * PS))) return rc;
-    if ((rc = dalloc(&h->facc3, npa * 18))) return rc;
+    Block b;
+    b.add(&h->ps, npa * PS);
+    b.add(&h->ps_alt, npa * PS);
+    b.add(&h->facc3, npa * 18);
+    b.add(&h->nbr, npa * MAX_NEIGH);
+    b.add(&h->nbr_count, npa);
+    b.add(&h->nbr_xy, npa * 2);
+    if ((rc = b.commit(&h->blk_part))) return rc;
     h->facc = h->facc3;
-    if ((rc = dalloc(&h->nbr, npa * MAX_NEIGH))) return rc;
-    if ((rc = dalloc(&h->nbr_count, npa))) return rc;
-    if ((rc = dalloc(&h->nbr_xy, npa * 2))) return rc;
   }
   CK(cudaMemsetAsync(h->ps, 0, sizeof(double) * npa * PS, h->stream));
   CK(cudaMemsetAsync(h->facc3, 0, sizeof(unsigned long long) * npa * 18, h->stream));
@@ -510,16 +549,20 @@ int setup_particle_buffers(lbm_sim* h, int np, double dmax) {
   h->series_cap = series_cap;
   if (h->p.series_every > 0) {
     if (!keep_s) {
-      if ((rc = dalloc(&h->series, (size_t)h->series_cap * h->series_len))) return rc;
-      if ((rc = dalloc(&h->mass_acc, (size_t)h->series_cap))) return rc;
+      Block b;
+      b.add(&h->series, (size_t)h->series_cap * h->series_len);
+      b.add(&h->mass_acc, (size_t)h->series_cap);
+      if ((rc = b.commit(&h->blk_series))) {
+        h->series = nullptr;
+        return rc;
+      }
       h->series_pcap = 2 * h->series_cap;
+      const size_t pin_n = (size_t)h->series_pcap * h->series_len;
       if (cudaHostAlloc(reinterpret_cast<void**>(&h->series_pin),
-                        sizeof(double) * h->series_pcap * h->series_len, cudaHostAllocDefault) !=
-              cudaSuccess ||
-          cudaHostAlloc(reinterpret_cast<void**>(&h->mass_pin),
-                        sizeof(unsigned long long) * h->series_pcap, cudaHostAllocDefault) !=
-              cudaSuccess)
+                        sizeof(double) * (pin_n + h->series_pcap), cudaHostAllocDefault) !=
+          cudaSuccess)
         return LBM_E_NOMEM;
+      h->mass_pin = reinterpret_cast<unsigned long long*>(h->series_pin + pin_n);
     }
     CK(cudaMemsetAsync(h->mass_acc, 0, sizeof(unsigned long long) * h->series_cap, h->stream));
   }
@@ -553,19 +596,42 @@ int launch_tiles(lbm_sim* h) {
   return LBM_OK;
 }
 
+// Pinned staging for npad disks.
+int reserve_ps_pin(lbm_sim* h) {
+  const size_t n = (size_t)h->npad * (PS + 6);
+  if (h->ps_pin_n >= n) return LBM_OK;
+  double* p = nullptr;
+  if (cudaHostAlloc(reinterpret_cast<void**>(&p), n * sizeof(double), cudaHostAllocDefault) !=
+      cudaSuccess)
+    return LBM_E_NOMEM;
+  if (h->ps_pin && h->ps_pin != reinterpret_cast<double*>(h->status_pin + STATUS_PIN_HEAD))
+    cudaFreeHost(h->ps_pin);
+  h->ps_pin = p;
+  h->ps_pin_n = n;
+  return LBM_OK;
+}
+
 // Particle records with FORCE of the last lattice step: while the
 // accumulators hold it (the next particle kernel decodes them on the
-// device), decode them here the same way.
+// device), decode them here the same way.  Refreshes the status too: three
+// copies to pinned memory and one wait.
 int read_particles(lbm_sim* h, std::vector<double>& buf) {
   const size_t npad = (size_t)h->npad;
-  std::vector<double> soa(npad * PS);
-  CK(d2h(h, soa.data(), h->ps, soa.size() * sizeof(double)));
+  int rc = reserve_ps_pin(h);
+  if (rc) return rc;
+  const bool force = h->partials_valid && h->np > 0;
+  double* soa = h->ps_pin;
+  const unsigned long long* acc = reinterpret_cast<unsigned long long*>(soa + npad * PS);
+  CK(cudaMemcpyAsync(soa, h->ps, npad * PS * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+  if (force)
+    CK(cudaMemcpyAsync(soa + npad * PS, h->facc, npad * 6 * sizeof(double),
+                       cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaMemcpyAsync(h->h_status, h->d_status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
   buf.assign((size_t)std::max(h->np, 1) * PS, 0.0);
   for (int i = 0; i < h->np; ++i)
     for (int f = 0; f < PS; ++f) buf[(size_t)i * PS + f] = soa[(size_t)f * npad + i];
-  if (h->partials_valid && h->np > 0) {
-    std::vector<unsigned long long> acc(npad * 6);
-    CK(d2h(h, acc.data(), h->facc, acc.size() * sizeof(unsigned long long)));
+  if (force) {
     for (int i = 0; i < h->np; ++i) {
       double* P = &buf[(size_t)i * PS];
       P[P_FX] = decode_force(acc[i], acc[npad + i]);
@@ -584,15 +650,8 @@ int read_particles(lbm_sim* h, std::vector<double>& buf) {
 int write_particles(lbm_sim* h, const std::vector<double>& buf) {
   const size_t npad = (size_t)h->npad;
   const size_t n = npad * PS;
-  if (h->ps_pin_n < n) {
-    if (h->ps_pin) cudaFreeHost(h->ps_pin);
-    h->ps_pin = nullptr;
-    h->ps_pin_n = 0;
-    if (cudaHostAlloc(reinterpret_cast<void**>(&h->ps_pin), n * sizeof(double),
-                      cudaHostAllocDefault) != cudaSuccess)
-      return LBM_E_NOMEM;
-    h->ps_pin_n = n;
-  }
+  const int rc = reserve_ps_pin(h);
+  if (rc) return rc;
   double* soa = h->ps_pin;
   std::fill(soa, soa + n, 0.0);
   for (int i = 0; i < h->np; ++i)
@@ -760,37 +819,19 @@ void destroy_buffers(lbm_sim* h) {
   if (h->adj_rs) cudaStreamSynchronize(h->adj_rs);
   for (cudaEvent_t e : h->ev) cudaEventDestroy(e);
   h->ev.clear();
-  for (int b = 0; b < 2; ++b) {
-    dfree(h->f[b]);
-    dfree(h->om[b]);
-    dfree(h->pm[b]);
-  }
-  dfree(h->rec);
-  dfree(h->ring);
-  dfree(h->ps); dfree(h->ps_alt); dfree(h->facc3); dfree(h->steps_bar);
-  dfree(h->nbr); dfree(h->nbr_count); dfree(h->nbr_xy);
-  dfree(h->tile_count); dfree(h->tile_list); dfree(h->tile_cur); dfree(h->pair_rebuild);
-  dfree(h->tile_order); dfree(h->n_unlisted); dfree(h->work_ctr);
-  dfree(h->rec_slot);
-  dfree(h->mass_acc);
-  dfree(h->d_kk); dfree(h->stale_dpw2);
-  dfree(h->series); dfree(h->out); dfree(h->out_f); dfree(h->d_status);
-  dfree(h->u0); dfree(h->err_part);
+  dfree(h->blk); dfree(h->blk_part); dfree(h->blk_series);
+  dfree(h->out_f); dfree(h->u0); dfree(h->err_part);
   if (h->series_pin) cudaFreeHost(h->series_pin);
-  if (h->mass_pin) cudaFreeHost(h->mass_pin);
-  if (h->ps_pin) cudaFreeHost(h->ps_pin);
+  if (h->ps_pin && h->ps_pin != reinterpret_cast<double*>(h->status_pin + STATUS_PIN_HEAD))
+    cudaFreeHost(h->ps_pin);
   for (const auto& b : h->series_pending) cudaEventDestroy(b.ev);
   for (cudaEvent_t e : h->series_ev_free) cudaEventDestroy(e);
   dfree(h->adj_slots); dfree(h->adj_ck); dfree(h->adj_ckp); dfree(h->adj_hist);
-  for (int b = 0; b < 2; ++b) {
-    dfree(h->adj_a[b]);
-    dfree(h->adj_w[b]);
-  }
-  dfree(h->adj_state); dfree(h->adj_p); dfree(h->adj_h); dfree(h->adj_rho); dfree(h->adj_g);
+  dfree(h->blk_adj); dfree(h->blk_adj_np);
   for (cudaEvent_t e : h->adj_ev)
     if (e) cudaEventDestroy(e);
   if (h->adj_rs) cudaStreamDestroy(h->adj_rs);
-  if (h->h_status) cudaFreeHost(h->h_status);
+  if (h->status_pin) cudaFreeHost(h->status_pin);
   if (h->copy_stream) cudaStreamDestroy(h->copy_stream);
   if (h->copy_fork) cudaEventDestroy(h->copy_fork);
   if (h->stream) cudaStreamDestroy(h->stream);
@@ -911,9 +952,11 @@ int enqueue_steps(lbm_sim* h, int left, int* done) {
   q.decode0 = h->partials_valid ? 1 : 0;
   const LatticeArgs a = lattice_args(h);
   const ParticleArgs pa = particle_args(h);
-  CK(cudaMemsetAsync(h->steps_bar, 0, sizeof(unsigned), h->stream));
-  CK(h->prec == LBM_FP64 ? launch_steps_fp64(a, pa, q, h->stream)
-                         : launch_steps_fp32(a, pa, q, h->stream));
+  int grid = 0;
+  q.bar0 = h->steps_bar_base;
+  CK(h->prec == LBM_FP64 ? launch_steps_fp64(a, pa, q, h->stream, &grid)
+                         : launch_steps_fp32(a, pa, q, h->stream, &grid));
+  h->steps_bar_base += (unsigned)(n - 1) * (unsigned)grid;
   h->kk += n;
   h->cur ^= n & 1;
   std::swap(h->ps, h->ps_alt);
@@ -1123,48 +1166,53 @@ int lbm_create(const lbm_params* pin, lbm_sim** out) {
       cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&h->copy_fork, cudaEventDisableTiming) != cudaSuccess)
     return fail(LBM_E_CUDA);
-  if (cudaHostAlloc(reinterpret_cast<void**>(&h->h_status), sizeof(int), cudaHostAllocDefault) !=
-      cudaSuccess)
+  const size_t pin0 = (size_t)32 * (PS + 6);  // ps_pin for up to 32 disks
+  if (cudaHostAlloc(reinterpret_cast<void**>(&h->status_pin),
+                    STATUS_PIN_HEAD + pin0 * sizeof(double), cudaHostAllocDefault) != cudaSuccess)
     return fail(LBM_E_NOMEM);
+  h->h_status = reinterpret_cast<int*>(h->status_pin);
+  h->ps_pin = reinterpret_cast<double*>(h->status_pin + STATUS_PIN_HEAD);
+  h->ps_pin_n = pin0;
   *h->h_status = 0;
-  if ((rc = dalloc(&h->d_status, 1))) return fail(rc);
-  cudaMemsetAsync(h->d_status, 0, sizeof(int), h->stream);
   const size_t fbytes = (size_t)9 * h->g.plane * h->esz;
-  for (int b = 0; b < 2; ++b) {
-    if (cudaMalloc(&h->f[b], fbytes) != cudaSuccess) return fail(LBM_E_NOMEM);
-    if (m.bingham && cudaMalloc(&h->om[b], (size_t)h->g.plane * h->esz) != cudaSuccess)
-      return fail(LBM_E_NOMEM);
-    if (m.bgk && m.bingham && cudaMalloc(&h->pm[b], (size_t)3 * h->g.plane * h->esz) != cudaSuccess)
-      return fail(LBM_E_NOMEM);
-  }
-  if (m.record_stress &&
-      cudaMalloc(&h->rec, (size_t)2 * 4 * h->g.plane * h->esz) != cudaSuccess)
-    return fail(LBM_E_NOMEM);
-  if (p.bc == LBM_BC_EQUILIBRIUM) {
-    h->ring_n = 2 * (p.nx + 1) + 2 * (p.ny + 1);
-    const size_t rb = (size_t)2 * 3 * h->ring_n * h->esz;
-    if (cudaMalloc(&h->ring, rb) != cudaSuccess) return fail(LBM_E_NOMEM);
-    cudaMemsetAsync(h->ring, 0, rb, h->stream);
-  }
-  if ((rc = make_tensor_maps(h))) return fail(rc);
+  const size_t pbytes = (size_t)h->g.plane * h->esz;
   const int ntiles = h->g.ltx * h->g.lty;
-  if ((rc = dalloc(&h->tile_count, (size_t)2 * ntiles))) return fail(rc);
-  if ((rc = dalloc(&h->tile_list, (size_t)2 * ntiles * h->tile_cap))) return fail(rc);
-  if ((rc = dalloc(&h->tile_cur, 2))) return fail(rc);
-  if ((rc = dalloc(&h->tile_order, (size_t)4 * ntiles))) return fail(rc);
-  if ((rc = dalloc(&h->n_unlisted, 2))) return fail(rc);
-  if ((rc = dalloc(&h->work_ctr, 2))) return fail(rc);
+  h->ring_n = p.bc == LBM_BC_EQUILIBRIUM ? 2 * (p.nx + 1) + 2 * (p.ny + 1) : 0;
+  const size_t rb = (size_t)2 * 3 * h->ring_n * h->esz;
+  {
+    Block b;
+    auto bytes = [&](void** q, size_t n) { b.add(reinterpret_cast<unsigned char**>(q), n); };
+    for (int k = 0; k < 2; ++k) {
+      bytes(&h->f[k], fbytes);
+      if (m.bingham) bytes(&h->om[k], pbytes);
+      if (m.bgk && m.bingham) bytes(&h->pm[k], 3 * pbytes);
+    }
+    if (m.record_stress) bytes(&h->rec, 8 * pbytes);
+    if (h->ring_n) bytes(&h->ring, rb);
+    b.add(&h->tile_count, (size_t)2 * ntiles);
+    b.add(&h->tile_list, (size_t)2 * ntiles * h->tile_cap);
+    b.add(&h->tile_cur, 2);
+    b.add(&h->tile_order, (size_t)4 * ntiles);
+    b.add(&h->n_unlisted, 2);
+    b.add(&h->work_ctr, 2);
+    b.add(&h->pair_rebuild, 1);
+    b.add(&h->rec_slot, 1);
+    b.add(&h->d_kk, 1);
+    b.add(&h->stale_dpw2, 2);
+    b.add(&h->steps_bar, 1);
+    b.add(&h->d_status, 1);
+    b.add(&h->out, (size_t)NOUT * nodes(h));
+    if ((rc = b.commit(&h->blk))) return fail(rc);
+  }
+  h->stale_dpw = h->stale_dpw2;
+  cudaMemsetAsync(h->d_status, 0, sizeof(int), h->stream);
+  cudaMemsetAsync(h->steps_bar, 0, sizeof(unsigned), h->stream);
+  if (h->ring) cudaMemsetAsync(h->ring, 0, rb, h->stream);
+  if ((rc = make_tensor_maps(h))) return fail(rc);
   cudaMemsetAsync(h->work_ctr, 0, 2 * sizeof(int), h->stream);
-  if ((rc = dalloc(&h->pair_rebuild, 1))) return fail(rc);
-  if ((rc = dalloc(&h->rec_slot, 1))) return fail(rc);
   cudaMemsetAsync(h->rec_slot, 0xff, sizeof(int), h->stream);
   cudaMemsetAsync(h->tile_cur, 0, 2 * sizeof(int), h->stream);
   cudaMemsetAsync(h->pair_rebuild, 0, sizeof(int), h->stream);
-  if ((rc = dalloc(&h->d_kk, 1))) return fail(rc);
-  if ((rc = dalloc(&h->stale_dpw2, 2))) return fail(rc);
-  h->stale_dpw = h->stale_dpw2;
-  if ((rc = dalloc(&h->steps_bar, 1))) return fail(rc);
-  if ((rc = dalloc(&h->out, (size_t)NOUT * nodes(h)))) return fail(rc);
   cudaMemsetAsync(h->f[0], 0, fbytes, h->stream);
   cudaMemsetAsync(h->f[1], 0, fbytes, h->stream);
   cudaMemsetAsync(h->tile_count, 0, sizeof(int) * 2 * ntiles, h->stream);
@@ -1273,7 +1321,7 @@ int lbm_get_particles(lbm_sim* h, double* out) {
     r[11] = P[P_FHX]; r[12] = P[P_FHY]; r[13] = P[P_FHT];
     r[14] = P[P_M]; r[15] = P[P_I];
   }
-  return refreshed_status(h);
+  return sticky_status(h);  // read with the records
 }
 
 int lbm_get_field(lbm_sim* h, int32_t which, double* out) {
@@ -1634,31 +1682,45 @@ int adj_reserve(lbm_sim* h, int nslots, int nck, long long nhist) {
   if (nhist > h->adj_nhist || h->adj_npad != h->npad) {
     dfree(h->adj_hist);
     h->adj_nhist = 0;
-    if ((rc = dalloc(&h->adj_hist, (size_t)nhist * PS * h->npad))) return rc;
+    // the records, then the objective's value of each step
+    if ((rc = dalloc(&h->adj_hist, (size_t)nhist * (PS * h->npad + 1)))) return rc;
     h->adj_nhist = nhist;
   }
   if (!h->adj_a[0]) {
+    Block k;
     for (int b = 0; b < 2; ++b) {
-      if ((rc = dalloc(reinterpret_cast<unsigned char**>(&h->adj_a[b]), 9 * h->g.plane * h->esz)))
-        return rc;
-      if ((rc = dalloc(reinterpret_cast<unsigned char**>(&h->adj_w[b]), h->g.plane * h->esz)))
-        return rc;
+      k.add(reinterpret_cast<unsigned char**>(&h->adj_a[b]), 9 * h->g.plane * h->esz);
+      k.add(reinterpret_cast<unsigned char**>(&h->adj_w[b]), h->g.plane * h->esz);
     }
-    if ((rc = dalloc(&h->adj_g, (size_t)2 * h->g.nbx * h->g.nby))) return rc;
+    k.add(&h->adj_g, (size_t)2 * h->g.nbx * h->g.nby);
+    if ((rc = k.commit(&h->blk_adj))) {
+      h->adj_a[0] = nullptr;
+      return rc;
+    }
   }
   if (!h->adj_rs) {
     CK(cudaStreamCreateWithFlags(&h->adj_rs, cudaStreamNonBlocking));
     for (cudaEvent_t& e : h->adj_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   }
   if (h->adj_npad != h->npad) {
-    dfree(h->adj_state); dfree(h->adj_p); dfree(h->adj_h); dfree(h->adj_rho);
+    dfree(h->blk_adj_np);
+    h->blk_adj_np = nullptr;
     const size_t np = (size_t)h->npad;
-    if ((rc = dalloc(&h->adj_state, 8 * np)) || (rc = dalloc(&h->adj_p, 5 * np)) ||
-        (rc = dalloc(&h->adj_h, 3 * np)) || (rc = dalloc(&h->adj_rho, np)))
-      return rc;
+    Block k;
+    k.add(&h->adj_state, 8 * np);
+    k.add(&h->adj_p, 5 * np);
+    k.add(&h->adj_h, 3 * np);
+    k.add(&h->adj_rho, np);
+    if ((rc = k.commit(&h->blk_adj_np))) return rc;
     h->adj_npad = h->npad;
   }
   return LBM_OK;
+}
+
+// out[k] = src[k * stride]: one field of one disk's records, every step.
+__global__ void k_pick(const double* src, size_t stride, int n, double* out) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < n) out[k] = src[(size_t)k * stride];
 }
 
 // Small state (records, FORCE sums, D_PW) into / out of checkpoint entry c.
@@ -1918,9 +1980,17 @@ extern "C" int lbm_adjoint(lbm_sim* h, const lbm_objective* obj, double* value, 
   CK(d2h(h, sv.data(), h->adj_state, sv.size() * sizeof(double)));
   CK(d2h(h, rv.data(), h->adj_rho, rv.size() * sizeof(double)));
   CK(d2h(h, gv.data(), h->adj_g, gv.size() * sizeof(double)));
-  std::vector<double> hist((size_t)(N + 1) * rec);
-  CK(d2h(h, hist.data(), h->adj_hist, hist.size() * sizeof(double)));
-  CK(cudaStreamSynchronize(h->stream));
+  const int field = comp == LBM_OBJ_X ? P_X : comp == LBM_OBJ_Y ? P_Y : comp == LBM_OBJ_U ? P_U
+                  : comp == LBM_OBJ_V ? P_V : P_W;
+  const int nval = (int)(obj->n1 - obj->n0 + 1);
+  std::vector<double> val((size_t)nval);
+  {
+    double* dv = h->adj_hist + (size_t)h->adj_nhist * rec;
+    k_pick<<<(nval + 255) / 256, 256, 0, h->stream>>>(
+        h->adj_hist + rec * obj->n0 + (size_t)field * np + obj->particle, rec, nval, dv);
+    CK(cudaGetLastError());
+    CK(d2h(h, val.data(), dv, val.size() * sizeof(double)));
+  }
   double gnu = 0.0, gty = 0.0;
   for (size_t b = 0; b < gv.size(); b += 2) {
     gnu += gv[b];
@@ -1934,11 +2004,8 @@ extern "C" int lbm_adjoint(lbm_sim* h, const lbm_objective* obj, double* value, 
     grads[LBM_GRAD_HEAD + LBM_GRAD_PER * q + 2] = sv[np + q];
   }
   if (value) {
-    const int field = comp == LBM_OBJ_X ? P_X : comp == LBM_OBJ_Y ? P_Y : comp == LBM_OBJ_U ? P_U
-                    : comp == LBM_OBJ_V ? P_V : P_W;
     double s = 0.0;
-    for (long long n = obj->n0; n <= obj->n1; ++n)
-      s += hist[rec * n + (size_t)field * np + obj->particle];
+    for (const double v : val) s += v;
     *value = s / (double)(obj->n1 - obj->n0 + 1);
   }
   return refreshed_status(h);

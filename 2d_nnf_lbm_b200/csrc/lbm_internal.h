@@ -211,7 +211,9 @@ struct LatticeArgs {
   int initial;           // 1: state is INITIALIZE (rho0, u=0, G=0)
 };
 
-// Several time steps of a small simulation in one launch (lbm_steps.cuh).
+// Several time steps of a small simulation in one launch (lbm_steps.cuh);
+// launch_steps_* set *grid to the blocks launched, each of which arrives at
+// the barrier nsteps - 1 times.
 constexpr int STEPS_MAX_DISKS = 256;
 struct StepsArgs {
   void* f[2];                // step s (1..nsteps) reads f[(s-1)&1], writes f[s&1]
@@ -221,15 +223,16 @@ struct StepsArgs {
   int facc0;
   double* stale;             // [2]: D_PW, read at stale0, written at stale0 ^ 1
   int stale0;
-  unsigned* bar;             // grid barrier, zero at the start
+  unsigned* bar;             // grid barrier, counts up for the handle's life
+  unsigned bar0;             // its count before the launch
   long long kk0;             // steps done before the launch
   int nsteps;
   int decode0;               // the accumulators hold FORCE of step kk0
 };
 cudaError_t launch_steps_fp64(const LatticeArgs& a, const ParticleArgs& p, const StepsArgs& q,
-                              cudaStream_t s);
+                              cudaStream_t s, int* grid);
 cudaError_t launch_steps_fp32(const LatticeArgs& a, const ParticleArgs& p, const StepsArgs& q,
-                              cudaStream_t s);
+                              cudaStream_t s, int* grid);
 
 // Launchers (defined in lbm_fp64.cu / lbm_fp32.cu).
 cudaError_t launch_init_fp64(const LatticeArgs& a, cudaStream_t s);

@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(STEPS_TPB, 1)
     if (tid == STEPS_TPB - 32) {
       S.next = S.next_late = S.n_late = 0;
       steps_arrive(q.bar);
-      if (!steps_wait(q.bar, (unsigned)s * gridDim.x, a.status)) S.stop = 1;
+      if (!steps_wait(q.bar, q.bar0 + (unsigned)s * gridDim.x, a.status)) S.stop = 1;
     }
     if (disk_warp) steps_disk_terms(p, S, kk + 1);
     __syncthreads();
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(STEPS_TPB, 1)
 
 template <class T>
 cudaError_t launch_steps(const LatticeArgs& a, const ParticleArgs& p, const StepsArgs& q,
-                         cudaStream_t s) {
+                         cudaStream_t s, int* grid_out) {
   const int sx = (a.m.bingham || a.m.record_stress) ? 1 : 0;
   void (*const kern)(const LatticeArgs, const ParticleArgs, const StepsArgs) =
       sx ? k_steps<T, true> : k_steps<T, false>;
@@ -438,6 +438,7 @@ cudaError_t launch_steps(const LatticeArgs& a, const ParticleArgs& p, const Step
   const long long nseg = (long long)((a.g.nx + 32) / 32) * (a.g.ny + 1);
   const int want = (int)((nseg + STEPS_WARPS - 1) / STEPS_WARPS);
   const int grid = want < sms ? want : sms;
+  *grid_out = grid;
   if ((nseg + grid - 1) / grid > STEPS_MAX_SEGS) return cudaErrorInvalidValue;
   LatticeArgs la = a;
   ParticleArgs pa = p;
