@@ -769,7 +769,7 @@ int encode_f_map(const lbm_sim* h, void* base, CUtensorMap* out, int tw = 0, int
   const cuuint64_t strides[2] = {(cuuint64_t)h->g.pitch * h->esz,
                                  (cuuint64_t)h->g.plane * h->esz};
   if (tw <= 0) tw = step_tile_width((int)h->esz);
-  if (rows <= 0) rows = step_box_rows((int)h->esz);
+  if (rows <= 0) rows = step_box_rows((int)h->esz, h->m.bingham || h->m.record_stress);
   const cuuint32_t box[3] = {(cuuint32_t)(tw + 2 * (16 / (int)h->esz)), (cuuint32_t)rows, 3};
   const cuuint32_t es[3] = {1, 1, 1};
   CUresult r = enc(out, h->esz == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
@@ -792,7 +792,7 @@ int encode_om_map(const lbm_sim* h, void* base, CUtensorMap* out, int tw = 0, in
   const cuuint64_t dims[2] = {(cuuint64_t)h->g.pitch, (cuuint64_t)(h->p.ny + 1)};
   const cuuint64_t strides[1] = {(cuuint64_t)h->g.pitch * h->esz};
   if (tw <= 0) tw = step_tile_width((int)h->esz);
-  if (rows <= 0) rows = step_box_rows((int)h->esz);
+  if (rows <= 0) rows = step_box_rows((int)h->esz, h->m.bingham || h->m.record_stress);
   const cuuint32_t box[2] = {(cuuint32_t)tw, (cuuint32_t)rows};
   const cuuint32_t es[2] = {1, 1};
   CUresult r = enc(out, h->esz == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,

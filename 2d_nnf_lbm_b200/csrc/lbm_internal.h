@@ -28,7 +28,7 @@ constexpr int TX = 32;
 constexpr int TY = 8;
 constexpr int TPB = TX * TY;
 // Particle candidate lists are kept per list tile of LTX x LTY nodes; a step
-// kernel tile (128 x 4 FP32 or 64 x 8 FP64 nodes) lies inside one list tile.
+// kernel tile (step_tile_nodes) lies inside one list tile.
 constexpr int LTX = 128;
 constexpr int LTY = 8;
 constexpr int MAX_TILE_CAND = 32;   // particles that may touch one tile
@@ -249,11 +249,20 @@ cudaError_t launch_restart_fp32(const LatticeArgs& a, cudaStream_t s);
 cudaError_t launch_bgk_step_fp64(const LatticeArgs& a, cudaStream_t s);
 cudaError_t launch_bgk_step_fp32(const LatticeArgs& a, cudaStream_t s);
 
-// TMA box of the step kernel: one tile row (128 FP32 / 64 FP64 nodes) plus
-// a 16-byte vector of halo on each side; 512 / row-width rows; one plane.
+// Tiles of the step kernel: rows of 128 (FP32) or 64 (FP64) nodes.  A block's
+// warps share a ring of staged tiles, and a tile's slot is refilled when its
+// last warp is done with it.  Without the strain rate a tile has 256 nodes
+// (four FP32 or two FP64 blocks per SM): with 512 (two, one) the warps wait
+// longer for each other (us per step, 512 / 256 nodes: sedimentation 1024 x
+// 2048 FP32 36.4 / 35.7, FP64 59.8 / 59.3, 1500 x 1000 FP64 40.1 / 39.2).
+// With it (STRESS: Bingham or stress record) it has 512: the node work is
+// longer, and a producer warp per 8 consumer warps takes issue slots from it
+// (viscoplastic 800 x 2400 FP64 59.0 / 61.5, FP32 36.7 / 36.9).
+__host__ __device__ constexpr int step_tile_nodes(bool stress) { return stress ? 512 : 256; }
+// TMA box of the step kernel: one tile row plus a 16-byte vector of halo on
+// each side; the tile's rows; one plane.
 inline int step_tile_width(int esz) { return esz == 8 ? 64 : 128; }
-inline int step_box_width(int esz) { return step_tile_width(esz) + 2 * (16 / esz); }
-inline int step_box_rows(int esz) { return 512 / (esz == 8 ? 64 : 128); }
+inline int step_box_rows(int esz, bool stress) { return step_tile_nodes(stress) / step_tile_width(esz); }
 
 // Particle kernel (lbm_particles.cu).
 cudaError_t launch_particles(const ParticleArgs& a, cudaStream_t s);

@@ -1038,26 +1038,32 @@ __global__ void __launch_bounds__(TPB, sizeof(T) == 8 ? LBM_MINB_F64 : LBM_MINB_
 // barrier is taken inside the loop.  Boxes that reach past the lattice are
 // zero-filled by the TMA unit; the nodes on the lattice edge gather their
 // populations from global memory with the boundary conditions instead.
-constexpr int STEP_CONSUMERS = 512;              // consumer threads (16 warps)
-constexpr int STEP_TPB = STEP_CONSUMERS + 32;    // + one producer warp
-
+//
 // TWv: nodes per tile row (the single-run kernel: 128 FP32, 64 FP64; the
-// batched kernel: 64, which leaves fewer threads idle on narrow lattices)
-template <class T, int TWv = (sizeof(T) == 8 ? 64 : 128)>
+// batched kernel: 64, which leaves fewer threads idle on narrow lattices).
+// NODES: nodes per tile, one consumer thread each (step_tile_nodes).
+template <class T, int TWv, int NODESv>
 struct Stage {
   static constexpr int H = 16 / (int)sizeof(T);               // halo: one 16-byte vector
   static constexpr int TW = TWv;                              // nodes per tile row
-  static constexpr int TR = STEP_CONSUMERS / TW;              // tile rows (8 or 4)
+  static constexpr int CONSUMERS = NODESv;                    // consumer threads
+  static constexpr int TPB = CONSUMERS + 32;                  // + one producer warp
+  static constexpr int TR = CONSUMERS / TW;                   // tile rows
   static constexpr int BW = TW + 2 * H;                       // box width (544 bytes)
   static constexpr int PLANE = TR * BW;                       // elements per plane box
-  static constexpr int BYTES = 9 * PLANE * (int)sizeof(T);     // the population boxes
+  // the three boxes of three planes, each on a 128-byte boundary (a TMA
+  // destination), in elements; the bytes they bring
+  static constexpr int GROUP = (3 * PLANE * (int)sizeof(T) + 127) / 128 * 128 / (int)sizeof(T);
+  static constexpr int BYTES = 9 * PLANE * (int)sizeof(T);
   // a Bingham model's node omega of the tile, one box without halo after
   // the populations (a global load per node on the collision's path otherwise)
+  static constexpr int OM_OFF = 3 * GROUP * (int)sizeof(T);
   static constexpr int OM_BYTES = TR * TW * (int)sizeof(T);
-  static constexpr int SLOT = BYTES + OM_BYTES;                // one stage
+  static constexpr int SLOT = OM_OFF + OM_BYTES;               // one stage
+  static_assert(OM_OFF % 128 == 0 && SLOT % 128 == 0, "TMA destinations");
   // offset of population k of a node from its column in the stage
   __host__ __device__ static constexpr int off(int k) {
-    return plane_of(k) * PLANE + ((k == 1 || k == 5 || k == 8) ? -1 : (k == 3 || k == 6 || k == 7) ? 1 : 0);
+    return plane_of(k) / 3 * GROUP + plane_of(k) % 3 * PLANE + ((k == 1 || k == 5 || k == 8) ? -1 : (k == 3 || k == 6 || k == 7) ? 1 : 0);
   }
 };
 
@@ -1095,7 +1101,11 @@ struct TileCand {
   __device__ __forceinline__ unsigned long long* facc(const LatticeArgs& a) const { return a.facc; }
 };
 
-template <class T, class ST = Stage<T>>
+// The single-run kernel's tiles.
+template <class T, bool STRESS>
+using StepStage = Stage<T, (sizeof(T) == 8 ? 64 : 128), step_tile_nodes(STRESS)>;
+
+template <class T, class ST>
 constexpr int step_smem() {
   return NSTAGE * ST::SLOT + 2 * 8 * NSTAGE + 64 + NSTAGE * (int)sizeof(TileCand);
 }
@@ -1119,7 +1129,7 @@ __device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
 }
 
-template <class T, class ST = Stage<T>>
+template <class T, class ST>
 __device__ __forceinline__ void tma_tile(const CUtensorMap* tm, uint32_t dst, uint32_t mbar,
                                          int bx, int by) {
   const int x = bx * ST::TW - ST::H;  // a multiple of H: 16-byte aligned
@@ -1128,7 +1138,7 @@ __device__ __forceinline__ void tma_tile(const CUtensorMap* tm, uint32_t dst, ui
 #pragma unroll
   for (int gq = 0; gq < 3; ++gq) {
     const int cy = gq == 0 ? 0 : (gq == 1 ? 1 : -1);
-    const uint32_t d = dst + (uint32_t)(3 * gq * ST::PLANE * (int)sizeof(T));
+    const uint32_t d = dst + (uint32_t)(gq * ST::GROUP * (int)sizeof(T));
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes "
         "[%0], [%1, {%2, %3, %4}], [%5];" ::"r"(d),
@@ -1139,7 +1149,7 @@ __device__ __forceinline__ void tma_tile(const CUtensorMap* tm, uint32_t dst, ui
 
 // The node omega of tile (bx, by) of a Bingham model: one 2-D box of TR
 // rows x TW nodes, no halo (x = bx * TW is a multiple of 16 bytes).
-template <class T, class ST = Stage<T>>
+template <class T, class ST>
 __device__ __forceinline__ void tma_omega(const CUtensorMap* tm, uint32_t dst, uint32_t mbar,
                                           int bx, int by) {
   asm volatile(
@@ -1207,8 +1217,8 @@ __device__ __forceinline__ void cand_copy(const LatticeArgs& a, CandList c, int 
   }
 }
 
-#ifndef LBM_STEP_MINB_F32
-#define LBM_STEP_MINB_F32 2
+#ifndef LBM_STEP_NODES_F32
+#define LBM_STEP_NODES_F32 1024
 #endif
 
 
@@ -1472,7 +1482,7 @@ __device__ __forceinline__ void step_body(const LatticeArgs& a, const CUtensorMa
                                           const CUtensorMap& tmo) {
   constexpr bool F64 = sizeof(T) == 8;
   constexpr uint32_t WAIT = 1u << 20;
-  using ST = Stage<T>;
+  using ST = StepStage<T, STRESS>;
   extern __shared__ __align__(128) unsigned char s_raw[];
   T* const stage_w = reinterpret_cast<T*>(s_raw);
   const uint32_t s_base = (uint32_t)__cvta_generic_to_shared(s_raw);
@@ -1487,7 +1497,7 @@ __device__ __forceinline__ void step_body(const LatticeArgs& a, const CUtensorMa
   const int ntx = (g.nx + 1 + ST::TW - 1) / ST::TW;
   const int nty = (g.ny + 1 + ST::TR - 1) / ST::TR;
 
-  if (tid == STEP_CONSUMERS) {  // the producer's descriptors, before its first issue
+  if (tid == ST::CONSUMERS) {  // the producer's descriptors, before its first issue
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tm)) : "memory");
     if (STRESS) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmo)) : "memory");
   }
@@ -1496,7 +1506,7 @@ __device__ __forceinline__ void step_body(const LatticeArgs& a, const CUtensorMa
       // "full": the TMA boxes (expect_tx) and the candidates, two arrivals
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(full0 + 8 * st) : "memory");
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(empty0 + 8 * st),
-                   "r"(STEP_CONSUMERS / 32)
+                   "r"(ST::CONSUMERS / 32)
                    : "memory");
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1506,7 +1516,7 @@ __device__ __forceinline__ void step_body(const LatticeArgs& a, const CUtensorMa
   // (it waits for this grid before it touches anything)
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-  if (warp == STEP_CONSUMERS / 32) {
+  if (warp == ST::CONSUMERS / 32) {
     // ================= producer warp =====================================
     // Tiles come from one queue shared by all CTAs (work_ctr[step & 1]): the
     // step tiles of the list tiles in tile_order of the previous step's list
@@ -1604,8 +1614,8 @@ __device__ __forceinline__ void step_body(const LatticeArgs& a, const CUtensorMa
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb),
                        "r"((uint32_t)(ST::BYTES + (om ? ST::OM_BYTES : 0)))
                        : "memory");
-          tma_tile<T>(&tm, s_base + sidx * ST::SLOT, fb, bx, by);
-          if (om) tma_omega<T>(&tmo, s_base + sidx * ST::SLOT + ST::BYTES, fb, bx, by);
+          tma_tile<T, ST>(&tm, s_base + sidx * ST::SLOT, fb, bx, by);
+          if (om) tma_omega<T, ST>(&tmo, s_base + sidx * ST::SLOT + ST::OM_OFF, fb, bx, by);
         }
       }
       // the candidates, while the boxes are in flight; second arrival
@@ -1700,7 +1710,7 @@ __device__ __forceinline__ void step_body(const LatticeArgs& a, const CUtensorMa
     T* const q = slot + tr * ST::BW + ST::H + tc;
     // the staged omega (none in a tile whose nodes all gather: bx * TW >= NX)
     const T* const omq = (STRESS && m.bingham && bx * ST::TW < g.nx)
-                             ? slot + ST::BYTES / (int)sizeof(T) + tid
+                             ? slot + ST::OM_OFF / (int)sizeof(T) + tid
                              : nullptr;
     NodeVals<T> v;
     node_stream<T, ST>(a, io, q, i, j, act, edge, v.f);
@@ -1724,10 +1734,12 @@ __device__ __forceinline__ void step_body(const LatticeArgs& a, const CUtensorMa
   }
 }
 
-// FP32: two CTAs per SM; FP64: one (with 17 warps, one SM sub-partition
-// holds 5 of them, which caps FP64 at 96 registers per thread).
+// 1024 nodes in flight per SM in FP32 (56 registers a thread), 512 in FP64
+// (96 registers).
 template <class T, bool STRESS>
-__global__ void __launch_bounds__(STEP_TPB, sizeof(T) == 8 ? 1 : LBM_STEP_MINB_F32)
+constexpr int STEP_MINB = (sizeof(T) == 8 ? 512 : LBM_STEP_NODES_F32) / step_tile_nodes(STRESS);
+template <class T, bool STRESS>
+__global__ void __launch_bounds__(StepStage<T, STRESS>::TPB, STEP_MINB<T, STRESS>)
     k_step(const LatticeArgs a, const __grid_constant__ CUtensorMap tm,
            const __grid_constant__ CUtensorMap tmo) {
   step_body<T, STRESS>(a, tm, tmo);
@@ -1735,42 +1747,40 @@ __global__ void __launch_bounds__(STEP_TPB, sizeof(T) == 8 ? 1 : LBM_STEP_MINB_F
 
 // tm: the population buffer read; tmo: its omega buffer (Bingham models;
 // any map otherwise, not read)
-template <class T>
+template <class T, bool STRESS>
 cudaError_t launch_step_tma(const LatticeArgs& a, const CUtensorMap* tm, const CUtensorMap* tmo,
                             cudaStream_t s) {
-  using ST = Stage<T>;
-  constexpr int SMEM = step_smem<T>();
-  const int sx = (a.m.bingham || a.m.record_stress) ? 1 : 0;
-  void (*const kern)(const LatticeArgs, const CUtensorMap, const CUtensorMap) =
-      sx ? k_step<T, true> : k_step<T, false>;
-  static int grid_of[2][64] = {};
+  using ST = StepStage<T, STRESS>;
+  constexpr int SMEM = step_smem<T, ST>();
+  void (*const kern)(const LatticeArgs, const CUtensorMap, const CUtensorMap) = k_step<T, STRESS>;
+  static int grid_of[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) dev = 0;
-  if (grid_of[sx][dev] == 0) {
+  if (grid_of[dev] == 0) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                              (int)cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
     int per_sm = 0, sms = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, STEP_TPB, SMEM);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, ST::TPB, SMEM);
     if (e != cudaSuccess) return e;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
     // one SM stays free for the particle kernel that runs beside the
     // particle-free tiles (it fills an SM's register file on its own)
-    grid_of[sx][dev] = (per_sm > 0 ? per_sm : 1) * (sms > 1 ? sms - 1 : 1);
+    grid_of[dev] = (per_sm > 0 ? per_sm : 1) * (sms > 1 ? sms - 1 : 1);
   }
   const int ntiles = ((a.g.nx + 1 + ST::TW - 1) / ST::TW) * ((a.g.ny + 1 + ST::TR - 1) / ST::TR);
-  const int grid = ntiles < grid_of[sx][dev] ? ntiles : grid_of[sx][dev];
+  const int grid = ntiles < grid_of[dev] ? ntiles : grid_of[dev];
   // Programmatic dependent launch: the kernel may start as soon as the
   // particle kernel before it on the stream allows (griddepcontrol.
   // launch_dependents); it waits for that kernel (griddepcontrol.wait) before
   // the tiles that need its results.
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(STEP_TPB);
+  cfg.blockDim = dim3(ST::TPB);
   cfg.dynamicSmemBytes = SMEM;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -1779,6 +1789,13 @@ cudaError_t launch_step_tma(const LatticeArgs& a, const CUtensorMap* tm, const C
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, a, *tm, *tmo);
+}
+
+template <class T>
+cudaError_t launch_step_tma(const LatticeArgs& a, const CUtensorMap* tm, const CUtensorMap* tmo,
+                            cudaStream_t s) {
+  return a.m.bingham || a.m.record_stress ? launch_step_tma<T, true>(a, tm, tmo, s)
+                                          : launch_step_tma<T, false>(a, tm, tmo, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1803,7 +1820,7 @@ cudaError_t launch_step_tma(const LatticeArgs& a, const CUtensorMap* tm, const C
 constexpr int BATCH_ARGS_SLOTS = 2 * NSTAGE;
 
 template <class T>
-using BatchStage = Stage<T, BATCH_TMA_TW>;
+using BatchStage = Stage<T, BATCH_TMA_TW, BATCH_TMA_TW * BATCH_TMA_TR>;
 static_assert(BatchStage<float>::TR == BATCH_TMA_TR && BatchStage<double>::TR == BATCH_TMA_TR,
               "batched TMA tile");
 
@@ -1813,7 +1830,7 @@ constexpr int batch_step_smem() {
 }
 
 template <class T, bool STRESS>
-__global__ void __launch_bounds__(STEP_TPB, sizeof(T) == 8 ? 1 : LBM_STEP_MINB_F32)
+__global__ void __launch_bounds__(BatchStage<T>::TPB, sizeof(T) == 8 ? 1 : 2)
     k_step_batch(const BatchSim* __restrict__ sims, int nsim,
                  const CUtensorMap* __restrict__ tmaps, long long total) {
   constexpr bool F64 = sizeof(T) == 8;
@@ -1837,7 +1854,7 @@ __global__ void __launch_bounds__(STEP_TPB, sizeof(T) == 8 ? 1 : LBM_STEP_MINB_F
     for (int st = 0; st < NSTAGE; ++st) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(full0 + 8 * st) : "memory");
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(empty0 + 8 * st),
-                   "r"(STEP_CONSUMERS / 32)
+                   "r"(ST::CONSUMERS / 32)
                    : "memory");
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1847,7 +1864,7 @@ __global__ void __launch_bounds__(STEP_TPB, sizeof(T) == 8 ? 1 : LBM_STEP_MINB_F
   const long long t_lo = (long long)blockIdx.x * per;
   const long long t_hi = t_lo + per < total ? t_lo + per : total;
 
-  if (warp == STEP_CONSUMERS / 32) {
+  if (warp == ST::CONSUMERS / 32) {
     // ================= producer warp =====================================
     int q = 0;
     if (lane == 0) {  // the last simulation whose first tile is <= t_lo
@@ -1944,7 +1961,7 @@ __global__ void __launch_bounds__(STEP_TPB, sizeof(T) == 8 ? 1 : LBM_STEP_MINB_F
                        "r"((uint32_t)(ST::BYTES + (om ? ST::OM_BYTES : 0)))
                        : "memory");
           tma_tile<T, ST>(tm, s_base + sidx * ST::SLOT, fb, bx, by);
-          if (om) tma_omega<T, ST>(tm + 2, s_base + sidx * ST::SLOT + ST::BYTES, fb, bx, by);
+          if (om) tma_omega<T, ST>(tm + 2, s_base + sidx * ST::SLOT + ST::OM_OFF, fb, bx, by);
         }
       }
       cand_copy(B.a, cl, bx, by, C, lane, fb);
@@ -2018,7 +2035,7 @@ __global__ void __launch_bounds__(STEP_TPB, sizeof(T) == 8 ? 1 : LBM_STEP_MINB_F
     T* const slot = stage_w + sidx * (ST::SLOT / (int)sizeof(T));
     T* const qp = slot + tr * ST::BW + ST::H + tc;
     const T* const omq = (STRESS && a.m.bingham && bx * ST::TW < g.nx)
-                             ? slot + ST::BYTES / (int)sizeof(T) + tid
+                             ? slot + ST::OM_OFF / (int)sizeof(T) + tid
                              : nullptr;
     NodeVals<T> v;
     node_stream<T, ST>(a, io, qp, i, j, act, edge, v.f);
@@ -2045,7 +2062,7 @@ cudaError_t batch_tma_prepare(int stress, int* blocks_per_sm) {
   e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                            (int)cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kern, STEP_TPB, SMEM);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kern, BatchStage<T>::TPB, SMEM);
 }
 
 template <class T>
@@ -2053,9 +2070,9 @@ cudaError_t launch_batch_tma(const BatchSim* sims, int nsim, const CUtensorMap* 
                              long long total, int stress, int grid, cudaStream_t s) {
   constexpr int SMEM = batch_step_smem<T>();
   if (stress)
-    k_step_batch<T, true><<<grid, STEP_TPB, SMEM, s>>>(sims, nsim, tmaps, total);
+    k_step_batch<T, true><<<grid, BatchStage<T>::TPB, SMEM, s>>>(sims, nsim, tmaps, total);
   else
-    k_step_batch<T, false><<<grid, STEP_TPB, SMEM, s>>>(sims, nsim, tmaps, total);
+    k_step_batch<T, false><<<grid, BatchStage<T>::TPB, SMEM, s>>>(sims, nsim, tmaps, total);
   return cudaGetLastError();
 }
 
