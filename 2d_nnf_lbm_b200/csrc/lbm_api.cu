@@ -138,7 +138,7 @@ struct lbm_sim {
   void* adj_a[2] = {nullptr, nullptr};  // dJ/dF, T[9 planes]
   void* adj_w[2] = {nullptr, nullptr};  // dJ/domega, T[plane]
   double* adj_state = nullptr;         // [8][npad]
-  double* adj_p = nullptr;             // [5][npad]
+  double* adj_p = nullptr;             // [3][5][npad] (k_adj_levels rotates them)
   double* adj_h = nullptr;             // [3][npad]
   double* adj_rho = nullptr;           // [npad]
   double* adj_g = nullptr;             // [blocks][2]
@@ -159,6 +159,7 @@ constexpr int STEPS_MAX_LAUNCH = 1024;  // time steps per launch of k_steps
 #endif
 constexpr long long STEPS_MAX_NODES = LBM_STEPS_MAX_NODES;
 constexpr long long STEPS_NODES_PER_DISK = 700;
+constexpr long long ADJ_LEVELS_MAX_NODES_F32 = 160000;
 
 int cuda_fail(cudaError_t e) {
   if (e == cudaErrorMemoryAllocation) return LBM_E_NOMEM;
@@ -920,7 +921,9 @@ bool steps_resident(const lbm_sim* h) {
 
 // Up to `left` time steps in one launch on the handle's stream; *done: how
 // many (bounded by the room in the history ring).
-int enqueue_steps(lbm_sim* h, int left, int* done) {
+// slots: the populations and omega are read from the 10-plane block there and
+// written to the blocks after it, one per step (the handle's own stay).
+int enqueue_steps(lbm_sim* h, int left, int* done, unsigned char* slots = nullptr) {
   const int every = h->p.series_every;
   int n = std::min(left, STEPS_MAX_LAUNCH);
   if (h->series && every > 0) {
@@ -936,9 +939,19 @@ int enqueue_steps(lbm_sim* h, int left, int* done) {
     }
   }
   StepsArgs q{};
-  for (int b = 0; b < 2; ++b) {
-    q.f[b] = h->f[h->cur ^ b];
-    q.om[b] = h->om[h->cur ^ b];
+  if (slots) {
+    const size_t pb = (size_t)h->g.plane * h->esz;
+    q.f = slots;
+    q.om = slots + 9 * pb;
+    q.f_stride = q.om_stride = 10 * (long long)pb;
+    q.mask = ~0;
+  } else {
+    auto bytes = [](void* p) { return static_cast<unsigned char*>(p); };
+    q.f = bytes(h->f[h->cur]);
+    q.om = bytes(h->om[h->cur]);
+    q.f_stride = bytes(h->f[h->cur ^ 1]) - q.f;
+    q.om_stride = bytes(h->om[h->cur ^ 1]) - q.om;
+    q.mask = 1;
   }
   q.ps[0] = h->ps;
   q.ps[1] = h->ps_alt;
@@ -958,7 +971,7 @@ int enqueue_steps(lbm_sim* h, int left, int* done) {
                          : launch_steps_fp32(a, pa, q, h->stream, &grid));
   h->steps_bar_base += (unsigned)(n - 1) * (unsigned)grid;
   h->kk += n;
-  h->cur ^= n & 1;
+  if (!slots) h->cur ^= n & 1;
   std::swap(h->ps, h->ps_alt);
   h->stale_dpw = h->stale_dpw2 + (q.stale0 ^ 1);
   h->facc = h->facc3 + (size_t)((q.facc0 + n) % 3) * 6 * h->npad;
@@ -1647,6 +1660,9 @@ const char* lbm_strerror(int code) {
 // kernel of the step before.  Two slot sets: the recompute of a segment runs
 // on a second stream while the level kernels of the segment after it run on
 // the handle's stream, so the two latency-bound kernel chains share the SMs.
+// A small lattice (adj_resident) takes the segments one after the other on the
+// handle's stream with one slot set: one launch of k_steps for a segment's
+// recompute, one of k_adj_levels for its levels.
 namespace {
 
 size_t adj_slot_bytes(const lbm_sim* h) { return (size_t)10 * h->g.plane * h->esz; }
@@ -1708,13 +1724,23 @@ int adj_reserve(lbm_sim* h, int nslots, int nck, long long nhist) {
     const size_t np = (size_t)h->npad;
     Block k;
     k.add(&h->adj_state, 8 * np);
-    k.add(&h->adj_p, 5 * np);
+    k.add(&h->adj_p, 3 * 5 * np);
     k.add(&h->adj_h, 3 * np);
     k.add(&h->adj_rho, np);
     if ((rc = k.commit(&h->blk_adj_np))) return rc;
     h->adj_npad = h->npad;
   }
   return LBM_OK;
+}
+
+// Whether an adjoint sweeps many levels per launch (k_adj_levels, with k_steps
+// for the forward pass and the recompute).  us per step of the whole gradient
+// at 200 steps, that way / one launch per kernel: FP64 101 x 301 28.0 / 32.4,
+// 201 x 501 34.7 / 35.3, 301 x 801 47.3 / 54.2, 351 x 1101 58.8 / 64.2; FP32
+// 101 x 301 26.3 / 30.5, 201 x 501 29.8 / 31.9 (Bingham 34.2 / 33.8), 301 x
+// 801 38.9 / 40 (46.4 / 41.9), 351 x 1101 47.8 / 42.8 (65.3 / 47.8).
+bool adj_resident(const lbm_sim* h) {
+  return steps_resident(h) && (h->prec == LBM_FP64 || nodes(h) <= ADJ_LEVELS_MAX_NODES_F32);
 }
 
 // out[k] = src[k * stride]: one field of one disk's records, every step.
@@ -1738,7 +1764,8 @@ cudaError_t adj_save_small(lbm_sim* h, int c) {
                          cudaMemcpyDeviceToDevice, h->stream);
 }
 
-int adj_load_small(lbm_sim* h, int c, long long kk, bool partials) {
+// tiles: the step kernel's lists are rebuilt for the loaded disks at once.
+int adj_load_small(lbm_sim* h, int c, long long kk, bool partials, bool tiles) {
   const double* d = h->adj_ckp + adj_ckp_len(h) * c;
   const size_t np = (size_t)h->npad;
   CK(cudaMemcpyAsync(h->ps, d, PS * np * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
@@ -1749,7 +1776,9 @@ int adj_load_small(lbm_sim* h, int c, long long kk, bool partials) {
   h->kk = kk;
   CK(launch_set_ll(h->d_kk, kk, h->stream));
   h->partials_valid = partials;
-  return launch_tiles(h);
+  if (tiles) return launch_tiles(h);
+  h->lists_stale = true;
+  return LBM_OK;
 }
 
 // f* and omega of the current state (f[cur], om[cur]) into a 10-plane block.
@@ -1779,13 +1808,14 @@ int adj_step_slots(lbm_sim* h, int s) {
   return LBM_OK;
 }
 
-AdjParticleArgs adj_particle_args(lbm_sim* h, const lbm_objective* obj, long long n) {
+// The particle adjoint of step n, whose lattice sums are in set ap of adj_p.
+AdjParticleArgs adj_particle_args(lbm_sim* h, const lbm_objective* obj, long long n, int ap = 0) {
   AdjParticleArgs q{};
   const size_t rec = (size_t)PS * h->npad;
   q.prev = h->adj_hist + rec * (n - 1);
   q.cur = h->adj_hist + rec * n;
   q.a_state = h->adj_state;
-  q.a_p = h->adj_p;
+  q.a_p = h->adj_p + (size_t)ap * 5 * h->npad;
   q.a_h = h->adj_h;
   q.a_rho = h->adj_rho;
   q.np = h->np;
@@ -1836,6 +1866,38 @@ cudaError_t adj_level(lbm_sim* h, long long n, const unsigned char* slot, const 
                              : launch_adj_lattice_fp32(a, h->stream, pdl);
 }
 
+// Levels hi .. lo of a small lattice, f*(lo) in the first of slots; ain, ap:
+// the current adjoint field and set of sums.
+int adj_levels(lbm_sim* h, const lbm_objective* obj, long long hi, long long lo,
+               const unsigned char* slots, int ain, bool have, int ap) {
+  AdjLevelsArgs a{};
+  a.g = h->g;
+  a.m = h->m;
+  a.p = adj_particle_args(h, obj, hi);
+  a.hist = h->adj_hist;
+  a.slots = slots;
+  a.slot_bytes = adj_slot_bytes(h);
+  for (int b = 0; b < 2; ++b) {
+    a.a[b] = h->adj_a[b];
+    a.aw[b] = h->adj_w[b];
+  }
+  a.in0 = ain;
+  a.have = have ? 1 : 0;
+  a.ap0 = ap;
+  a.n_hi = hi;
+  a.n_lo = lo;
+  a.gacc = h->adj_g;
+  a.kappa = 36.0 * h->p.d_mrt;
+  a.bar = h->steps_bar;
+  a.bar0 = h->steps_bar_base;
+  a.status = h->d_status;
+  int grid = 0;
+  CK(h->prec == LBM_FP64 ? launch_adj_levels_fp64(a, h->stream, &grid)
+                         : launch_adj_levels_fp32(a, h->stream, &grid));
+  h->steps_bar_base += (unsigned)(hi - lo) * (unsigned)grid;
+  return LBM_OK;
+}
+
 }  // namespace
 
 extern "C" int lbm_adjoint(lbm_sim* h, const lbm_objective* obj, double* value, double* grads) {
@@ -1865,7 +1927,8 @@ extern "C" int lbm_adjoint(lbm_sim* h, const lbm_objective* obj, double* value, 
                                           : std::max<long long>(1, std::llround(std::sqrt((double)N)));
   L = std::max<long long>(1, std::min<long long>(L, std::max<long long>(nlev, 1)));
   const int C = nlev > 0 ? (int)((nlev + L - 1) / L) : 0;
-  const int nsets = C >= 2 ? 2 : 1;
+  const bool resident = adj_resident(h);
+  const int nsets = C >= 2 && !resident ? 2 : 1;
   int rc = adj_reserve(h, nsets * (int)L, C, N + 1);
   if (rc) return rc;
   const size_t rec = (size_t)PS * h->npad;
@@ -1876,7 +1939,7 @@ extern "C" int lbm_adjoint(lbm_sim* h, const lbm_objective* obj, double* value, 
                      h->stream));
   std::vector<char> ck_partials(C + 1, 0);
   h->adj_record = true;  // the particle kernel stores each step's records
-  for (long long n = 1; n <= N && rc == LBM_OK; ++n) {
+  for (long long n = 1; n <= N && rc == LBM_OK;) {
     if ((n - 1) % L == 0 && (n - 1) / L < C) {
       const int c = (int)((n - 1) / L);
       cudaError_t e = adj_save_fields(h, h->adj_ck + sb * c);
@@ -1884,7 +1947,13 @@ extern "C" int lbm_adjoint(lbm_sim* h, const lbm_objective* obj, double* value, 
       if (e != cudaSuccess) rc = cuda_fail(e);
       ck_partials[c] = h->partials_valid ? 1 : 0;
     }
-    if (rc == LBM_OK) rc = enqueue_step(h);
+    int done = 1;
+    if (rc == LBM_OK) {
+      const long long upto = (n - 1) / L < C - 1 ? ((n - 1) / L + 1) * L : N;
+      rc = resident ? enqueue_steps(h, (int)std::min<long long>(upto - n + 1, INT32_MAX), &done)
+                    : enqueue_step(h);
+    }
+    n += done;
   }
   h->adj_record = false;
   if (rc) return rc;
@@ -1895,7 +1964,7 @@ extern "C" int lbm_adjoint(lbm_sim* h, const lbm_objective* obj, double* value, 
   // ---- reverse --------------------------------------------------------------
   const size_t np = (size_t)h->npad;
   CK(cudaMemsetAsync(h->adj_state, 0, 8 * np * sizeof(double), h->stream));
-  CK(cudaMemsetAsync(h->adj_p, 0, 5 * np * sizeof(double), h->stream));
+  CK(cudaMemsetAsync(h->adj_p, 0, 15 * np * sizeof(double), h->stream));
   CK(cudaMemsetAsync(h->adj_h, 0, 3 * np * sizeof(double), h->stream));
   CK(cudaMemsetAsync(h->adj_rho, 0, np * sizeof(double), h->stream));
   CK(cudaMemsetAsync(h->adj_g, 0, 2 * (size_t)h->g.nbx * h->g.nby * sizeof(double), h->stream));
@@ -1917,7 +1986,25 @@ extern "C" int lbm_adjoint(lbm_sim* h, const lbm_objective* obj, double* value, 
   CK(cudaStreamWaitEvent(h->adj_rs, h->adj_ev[4], 0));
   int ain = 0;
   bool have = false;
-  {
+  if (resident) {  // the same segments, one after the other on the handle's stream
+    int ap = 0;
+    for (int c = C - 1; c >= 0; --c) {
+      const long long t0 = (long long)c * L;
+      const long long hi = std::min<long long>(t0 + L, nlev);
+      CK(cudaMemcpyAsync(h->adj_slots, h->adj_ck + sb * c, sb, cudaMemcpyDeviceToDevice,
+                         h->stream));
+      if ((rc = adj_load_small(h, c, t0, ck_partials[c] != 0, false))) return rc;
+      for (int s = 0, done = 0; t0 + 1 + s < hi; s += done)
+        if ((rc = enqueue_steps(h, (int)(hi - t0 - 1) - s, &done, h->adj_slots + sb * s)))
+          return rc;
+      if ((rc = adj_levels(h, obj, hi, t0 + 1, h->adj_slots, ain, have, ap))) return rc;
+      have = true;
+      ain ^= (int)((hi - t0) & 1);
+      ap = (int)((ap + hi - t0 - 1) % 3);
+      CK(launch_adj_particles(adj_particle_args(h, obj, t0 + 1, ap), h->stream));
+      ap = (ap + 1) % 3;
+    }
+  } else {
     struct Join {
       lbm_sim* h;
       ~Join() {
@@ -1942,7 +2029,7 @@ extern "C" int lbm_adjoint(lbm_sim* h, const lbm_objective* obj, double* value, 
       const int base = set * (int)L;
       CK(cudaMemcpyAsync(h->adj_slots + sb * base, h->adj_ck + sb * c, sb,
                          cudaMemcpyDeviceToDevice, h->stream));
-      int r = adj_load_small(h, c, t0, ck_partials[c] != 0);
+      int r = adj_load_small(h, c, t0, ck_partials[c] != 0, true);
       for (int s = 0; r == LBM_OK && t0 + 1 + s < hi; ++s) r = adj_step_slots(h, base + s);
       if (r) return r;
       CK(cudaEventRecord(h->adj_ev[set], h->stream));
@@ -1973,7 +2060,7 @@ extern "C" int lbm_adjoint(lbm_sim* h, const lbm_objective* obj, double* value, 
   CK(adj_level(h, 0, nullptr, have ? h->adj_a[ain] : nullptr, have ? h->adj_w[ain] : nullptr,
                nullptr, nullptr, 1));
   // the handle back at step N
-  if ((rc = adj_load_small(h, C, N, final_partials))) return rc;
+  if ((rc = adj_load_small(h, C, N, final_partials, !resident))) return rc;
 
   // ---- results ----------------------------------------------------------------
   std::vector<double> sv(8 * np), rv(np), gv(2 * (size_t)h->g.nbx * h->g.nby);

@@ -216,8 +216,13 @@ struct LatticeArgs {
 // the barrier nsteps - 1 times.
 constexpr int STEPS_MAX_DISKS = 256;
 struct StepsArgs {
-  void* f[2];                // step s (1..nsteps) reads f[(s-1)&1], writes f[s&1]
-  void* om[2];
+  // step s (1..nsteps) reads the populations at f + ((s-1) & mask) * f_stride
+  // (bytes) and writes those at f + (s & mask) * f_stride; omega likewise.
+  // Two buffers in turn: mask 1; a buffer per step: mask ~0.
+  unsigned char* f;
+  unsigned char* om;
+  long long f_stride, om_stride;
+  int mask;
   double* ps[2];             // [PS][npad] disk state: read, and written at the end
   unsigned long long* facc;  // [3][6][npad]: step s adds to (facc0 + s) % 3
   int facc0;
@@ -324,16 +329,17 @@ cudaError_t launch_particles_batch(const ParticleArgs* args, int nsim, cudaStrea
 // step n+1 then maps (records n, FORCE(n)) to records n+1.
 constexpr int ADJ_MAX_PARTICLES = 64;
 
-// Adjoint field of the populations: a[k] is dJ/dF(k) of the populations
-// after streaming and boundary conditions, stored like f (plane_of(k) planes).
+// Adjoint field of the populations: a[k] is dJ/dr(k) of the pulled populations
+// before the boundary routine (adj_boundary in lbm_adjoint.cu), stored like f
+// (plane_of(k) planes).
 struct AdjLatticeArgs {
   Geometry g;
   Model m;
   const void* fs;       // f*(n) (T planes); unused at level 0
   const void* oms;      // omega(n) (T), Bingham
-  const void* a_in;     // dJ/dF(n+1) (T planes), null: zero
+  const void* a_in;     // adjoint field of level n+1 (T planes), null: zero
   const void* aw_in;    // dJ/domega(n+1) (T), null: zero
-  void* a_out;          // dJ/dF(n) (T planes); unused at level 0
+  void* a_out;          // adjoint field of level n (T planes); unused at level 0
   void* aw_out;         // dJ/domega(n) (T), Bingham
   const double* ps;     // particle records of step n, [PS][npad]
   const double* a_h;    // dJ/dFORCE(n), [3][npad] (x, y, torque)
@@ -361,6 +367,31 @@ struct AdjParticleArgs {
   int nx, ny;
 };
 
+// Levels n_hi .. n_lo (n_lo >= 1) of a small lattice in one launch, with the
+// particle adjoints of steps n_hi .. n_lo + 1 between them (those of n_hi + 1
+// before and of n_lo after it are launch_adj_particles').
+struct AdjLevelsArgs {
+  Geometry g;
+  Model m;
+  AdjParticleArgs p;           // prev, cur, n unused; a_p: [3][5][npad], see ap0
+  const double* hist;          // records of every step, [PS][npad] each
+  const unsigned char* slots;  // f*(n_lo), omega(n_lo); the next levels' after it
+  size_t slot_bytes;
+  void* a[2];                  // adjoint field, dJ/domega: read at in0 first (zero if
+  void* aw[2];                 // !have), the level after reads what this wrote
+  int in0, have;
+  int ap0;                     // the a_p set of level n_hi (l levels on: ap0 + l mod 3)
+  long long n_hi, n_lo;
+  double* gacc;                // as in AdjLatticeArgs
+  double kappa;
+  unsigned* bar;               // grid barrier, counts up
+  unsigned bar0;               // its count before the launch
+  int* status;
+};
+
+// *grid: blocks of the launch (each adds n_hi - n_lo to bar).
+cudaError_t launch_adj_levels_fp32(const AdjLevelsArgs& a, cudaStream_t s, int* grid);
+cudaError_t launch_adj_levels_fp64(const AdjLevelsArgs& a, cudaStream_t s, int* grid);
 // pdl: launch as a programmatic dependent of the previous kernel (which must
 // be the particle adjoint kernel: the lattice kernel waits for it only
 // before reading dJ/dFORCE and adding to a_p).

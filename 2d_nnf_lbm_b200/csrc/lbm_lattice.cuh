@@ -39,6 +39,23 @@ __device__ __forceinline__ double wexact(int k) {
   return k == 0 ? 4.0 / 9.0 : (k < 5 ? 1.0 / 9.0 : 1.0 / 36.0);
 }
 
+// Grid-wide barrier, in two halves, of the thread that keeps it (the others
+// wait at a block barrier before and after): the block's writes are visible
+// to every block that has passed it.
+__device__ __forceinline__ void grid_arrive(unsigned* bar) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+}
+// False if it did not complete within the limit.
+__device__ __forceinline__ bool grid_wait(const unsigned* bar, unsigned target, int* status) {
+  for (int it = 0; it < (1 << 22); ++it) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+    if ((int)(v - target) >= 0) return true;
+  }
+  atomicOr(status, ST_TIMEOUT);
+  return false;
+}
+
 // A load of data that other blocks write during the launch (CG: past the L1
 // cache), or an ordinary one.
 template <bool CG, class T>

@@ -71,23 +71,6 @@ struct BlockCand {
   __device__ __forceinline__ int id(int c) const { return S.idx[c]; }
 };
 
-// Grid-wide barrier, in two halves, of the thread that keeps it (the others
-// wait at a block barrier before and after): the block's writes are visible
-// to every block that has passed it.
-__device__ __forceinline__ void steps_arrive(unsigned* bar) {
-  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-}
-// False if it did not complete within the limit.
-__device__ __forceinline__ bool steps_wait(const unsigned* bar, unsigned target, int* status) {
-  for (int it = 0; it < (1 << 22); ++it) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-    if ((int)(v - target) >= 0) return true;
-  }
-  atomicOr(status, ST_TIMEOUT);
-  return false;
-}
-
 // Pair lists and the block's disk list from the centres at parity b (the
 // whole block calls it).
 static __device__ __noinline__ void steps_lists(const ParticleArgs& p, StepsShared& S, int b, int row0, int row1) {
@@ -300,8 +283,11 @@ __global__ void __launch_bounds__(STEPS_TPB, 1)
   for (int s = 1; s <= q.nsteps; ++s) {
     const long long kk = q.kk0 + s;
     const bool rec = p.series != nullptr && p.series_every > 0 && kk % p.series_every == 0;
-    const StepIO<T> io{static_cast<const T*>(q.f[(s - 1) & 1]), static_cast<T*>(q.f[s & 1]),
-                       static_cast<const T*>(q.om[(s - 1) & 1]), static_cast<T*>(q.om[s & 1]), kk};
+    const long long from = (s - 1) & q.mask, to = s & q.mask;
+    const StepIO<T> io{reinterpret_cast<const T*>(q.f + from * q.f_stride),
+                       reinterpret_cast<T*>(q.f + to * q.f_stride),
+                       reinterpret_cast<const T*>(q.om + from * q.om_stride),
+                       reinterpret_cast<T*>(q.om + to * q.om_stride), kk};
     unsigned long long* const facc = q.facc + (long long)((q.facc0 + s) % 3) * 6 * p.npad;
     long long mass_q = 0;
     // one segment of 32 nodes; nc listed disks at the centres of step kk
@@ -398,8 +384,8 @@ __global__ void __launch_bounds__(STEPS_TPB, 1)
     if (s == q.nsteps) break;
     if (tid == STEPS_TPB - 32) {
       S.next = S.next_late = S.n_late = 0;
-      steps_arrive(q.bar);
-      if (!steps_wait(q.bar, q.bar0 + (unsigned)s * gridDim.x, a.status)) S.stop = 1;
+      grid_arrive(q.bar);
+      if (!grid_wait(q.bar, q.bar0 + (unsigned)s * gridDim.x, a.status)) S.stop = 1;
     }
     if (disk_warp) steps_disk_terms(p, S, kk + 1);
     __syncthreads();

@@ -301,7 +301,8 @@ int32_t lbm_checked_build(void);
  * Device memory kept by the handle: ceil((n1 - 1) / L) checkpoints, two sets
  * of L slots (one set when there is a single segment), each 10 lattice
  * planes, L = checkpoint_every; a segment's recompute runs on a second
- * stream of the handle beside the reverse sweep of the segment after it.
+ * stream of the handle beside the reverse sweep of the segment after it (a
+ * small lattice takes one set of slots and the segments in turn).
  * The call returns when the sweep is done.
  * grads receives 2 + 3*np doubles:
  *   [LBM_GRAD_TAU_Y] dJ/dtau_y   [LBM_GRAD_NU] dJ/dnu (plastic viscosity)
