@@ -94,7 +94,8 @@ __device__ __forceinline__ double wall_force(const ParticleArgs& a, int iw, doub
       const Rn c = E_W * CIJ * (Rn(D) - W) / ZITA;
       f = (EPS_W * CIJ * (q * q) + c) * e / W;
     }
-    F[vert ? 1 : 0] = f.v;
+    if (vert) F[1] = f.v;
+    else F[0] = f.v;
   }
   return D_PW;
 }
