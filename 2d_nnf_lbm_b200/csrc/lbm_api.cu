@@ -5,6 +5,8 @@
 //   k_particles  repulsion, Newton-Euler update, history, tile lists
 //   k_step       stream + BC + macro + SPM + force sums + correction +
 //                collision of the next step (persistent, TMA-fed)
+// or, for a small lattice (steps_resident), one launch of k_steps for many
+// steps.
 // The post-collision populations live in a ping-pong pair: after step K,
 // f[cur] holds f*(K+1) and f[cur^1] holds f*(K), from which the output
 // kernel re-derives the fields of step K (F after BC, rho, u, G, PHI) on
@@ -908,12 +910,14 @@ int enqueue_step(lbm_sim* h) {
 }
 
 // Whether the handle steps several steps per launch (k_steps).  The line is
-// where the two ways take the same time (us per step, k_steps / the particle
-// and step kernels): FP64 201 x 601 7.7 / 11.2, 401 x 801 11.3 / 13.5, 501 x
-// 1001 16.2 / 15.7; FP32 6.8 / 10.6, 9.7 / 10.5, 12.4 / 11.9.  A step of k_steps grows faster with
-// the lattice (its blocks load by node, the step kernel by TMA tiles) and
-// with the disks (each block updates all of them): at 513 x 513 with 20 disks
-// 12.2 / 12.8 (FP64), with 200 disks 18.8 / 18.5.
+// where the two ways take about the same time (us per step, k_steps / the
+// particle and step kernels, a record every 10 steps): FP64 201 x 601 7.1 /
+// 9.5, 401 x 801 10.5 / 12.6, 501 x 1001 14.0 / 15.2, Bingham 361 x 1081 17.3 /
+// 18.4; FP32 6.2 / 9.0, 9.0 / 9.8, 11.5 / 11.2, 13.2 / 12.9.  A step of k_steps
+// grows faster with the lattice (its blocks load by node, the step kernel by
+// TMA tiles) and with the disks (each block updates all of them): at 513 x 513
+// with 100 disks 14.5 / 14.7 (FP64) and 12.4 / 13.0, with 200 disks 17.8 / 16.4
+// and 15.1 / 14.4.
 bool steps_resident(const lbm_sim* h) {
   return !h->prof && !h->m.bgk && h->np <= STEPS_MAX_DISKS &&
          nodes(h) + STEPS_NODES_PER_DISK * h->np <= STEPS_MAX_NODES;
@@ -1299,7 +1303,12 @@ int lbm_step(lbm_sim* h, int32_t nsteps) {
   cudaSetDevice(h->p.device);
   for (int32_t s = 0; s < nsteps;) {
     int n = 1;
-    int rc = steps_resident(h) ? enqueue_steps(h, nsteps - s, &n) : enqueue_step(h);
+    // A call of one step, with tile lists up to date: the two kernels.  k_steps
+    // sets itself up at each launch; a call of n steps and the read of the
+    // disks, us, k_steps / two kernels, 201 x 601: FP64 n = 1 43.7 / 37.3, n = 2
+    // 47.1 / 50.0, n = 4 62.9 / 67.6; FP32 43.3 / 34.2, 45.0 / 45.8, 57.1 / 58.5.
+    const bool one = nsteps == 1 && !h->lists_stale;
+    int rc = steps_resident(h) && !one ? enqueue_steps(h, nsteps - s, &n) : enqueue_step(h);
     if (rc) return rc;
     s += n;
   }

@@ -1,7 +1,8 @@
 // lbm_fp64.cu -- FP64 plain-population instantiation of the lattice kernel.
-// Built with --fmad=false: every product and sum rounds on its own, in the
-// reference's order, so the only differences from the FP64 oracle come from
-// sin() and from the order of the force reductions.
+// Built with --fmad=false: a product and a sum are fused only where the source
+// says fma, so the kernels that share an operation give the same bits.  The
+// differences from the FP64 oracle are the collision's rounding (macro64,
+// collide64), sin() and the order of the force reductions.
 #include "lbm_lattice.cuh"
 #include "lbm_steps.cuh"
 

@@ -17,10 +17,12 @@
 // particle, so results do not depend on block scheduling.
 //
 // Precision policies:
-//   double -- plain populations f, operation order of the reference; the TU
-//             is compiled with --fmad=false so products are not contracted.
+//   double -- plain populations f; density, velocity and the first moments in
+//             the operation order of the reference, the collision from shared
+//             sums (collide64).
 //   float  -- shifted populations h = f - w_k*rho0 in FP32, FP32 arithmetic;
 //             force/torque/mass reductions in FP64.
+// Both TUs are compiled with --fmad=false: what is fused is written as fma.
 #pragma once
 
 #include <cuda.h>

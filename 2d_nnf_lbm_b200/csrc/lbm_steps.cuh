@@ -1,15 +1,15 @@
 // lbm_steps.cuh -- several time steps of a small simulation in one launch.
 //
 // A small lattice does not fill the GPU for long: 201 x 601 nodes are two
-// passes of one 512-thread block per SM, and what a step took (11.2 us FP64,
-// 10.6 us FP32) was the chain of two dependent kernels, their start-up and
-// the particle kernel's own latency.  k_steps stays resident over many steps
+// passes of one 512-thread block per SM, and what a step takes in kernels of
+// its own (9.5 us FP64, 9.0 us FP32) is the chain of two dependent kernels,
+// their start-up and the particle kernel's own latency.  k_steps stays resident over many steps
 // (a cooperative launch, one block per SM): each block owns a contiguous range
 // of 32-node row segments, the populations stay in L2 (17 MB of the 126 MB at
 // that size), and the only synchronisation between blocks is one grid-wide
-// barrier per step.  It takes 7.7 us (FP64) and 6.8 us (FP32): about 2 us the
-// barrier, 1 us the disk's update, 0.6 us a history record every step, the
-// rest the node arithmetic.
+// barrier per step.  It takes 7.1 us (FP64) and 6.2 us (FP32): about 2 us the
+// barrier, 1 us the disk's update, the rest the node arithmetic; a history
+// record every step costs 0.6 us more.
 //
 // There is no particle kernel: every block holds the state of all disks in
 // shared memory and updates all of them, from the same inputs and so to the

@@ -133,3 +133,24 @@ def test_resident_handles_interleave(pkg, cases):
     assert np.array_equal(b.particles(), alone[1])
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("program,nx,ny,n,diam", [("c6", 32, 65, 1, 8.0), ("c3", 96, 131, 33, 8.0)])
+def test_calls_of_one_step_mix_with_longer_ones(pkg, cases, program, nx, ny, n, diam):
+    """A call of one step takes the two kernels while the tile lists are up to
+    date, the resident kernel after a longer call: FP64 bit for bit the same
+    as one call."""
+    p, pin = build(cases, program, nx, ny, n, diam, 0)
+    p.series_every = 0
+    got = []
+    for calls in ((40,), (1, 1, 1, 12, 1, 1, 2, 20, 1), (1,) * 40):
+        s = pkg.Simulation(p)
+        s.set_particles(pin)
+        for k in calls:
+            s.step(k)
+        assert s.kk == 40 and s.status() == 0
+        got.append(read_all(s))
+        s.close()
+    for g in got[1:]:
+        for k, w in got[0].items():
+            assert np.array_equal(g[k], w, equal_nan=True), k
