@@ -812,6 +812,9 @@ __global__ void __launch_bounds__(ADJ_MAX_PARTICLES) k_adj_particles(const AdjPa
 // gather and collision.
 constexpr int LEVELS_TPB = 512;
 constexpr int LEVELS_WARPS = LEVELS_TPB / 32;
+// Segments a block has at least (the gradient of 400 steps at 101 x 301 with 16
+// / 12 / 8 / 4, here and in k_steps: 9.8 / 9.35 / 9.2 / 9.3 ms FP64).
+constexpr int LEVELS_MIN_SEGS = 8;
 constexpr uint32_t LEVELS_WAIT = 1u << 22;  // polls of dJ/dFORCE before giving up
 
 template <class T>
@@ -1016,7 +1019,7 @@ cudaError_t launch_levels(const AdjLevelsArgs& a, cudaStream_t s, int* grid_out)
     return e;
   // one slot of gacc per block: never more blocks than nbx * nby
   const long long nseg = (long long)((a.g.nx + 32) / 32) * (a.g.ny + 1);
-  const long long want = std::min<long long>((nseg + LEVELS_WARPS - 1) / LEVELS_WARPS,
+  const long long want = std::min<long long>((nseg + LEVELS_MIN_SEGS - 1) / LEVELS_MIN_SEGS,
                                              (long long)a.g.nbx * a.g.nby);
   const int grid = (int)std::min<long long>(want, sms);
   *grid_out = grid;
