@@ -300,8 +300,10 @@ __device__ __forceinline__ void adj_macro(const Model& m, bool fluid, const T* m
   v.rho = (T)m.rho0;
   if (fluid) v.rho = (T)m.rho0 + mh[0];
   v.ir = (T)1 / v.rho;
-  v.upx = fluid ? mh[3] * v.ir : (T)0;
-  v.upy = fluid ? mh[5] * v.ir : (T)0;
+  // divided, not times 1/rho: the sums over a disk that cancel (dJ/dy0 of one
+  // between two nodes) show its last bit, 1e-5 of the entry in FP32
+  v.upx = fluid ? mh[3] / v.rho : (T)0;
+  v.upy = fluid ? mh[5] / v.rho : (T)0;
   v.win = -1;
   v.phw = v.dphw = v.usxw = v.usyw = (T)0;
 }
