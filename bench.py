@@ -66,7 +66,7 @@ FALLBACK_HBM_GBS = 6650.0
 # from ncu (dram__bytes_read.sum + dram__bytes_write.sum, one launch, cold);
 # captured with `ncu --set full -k regex:k_step -s 5 -c 1` on
 # `python bench.py --profile-run step-fp32 --steps 30` (summary under profiles/)
-K_STEP_FP32_TRAFFIC = {"bytes": 112485888.0, "captured_at": "0e24264"}
+K_STEP_FP32_TRAFFIC = {"bytes": 113035008.0, "captured_at": "fe9b19e"}
 PARTS = ("fp32", "fp64", "e2e", "trajectory", "viscoplastic", "adjoint", "batch", "cpu")
 
 
