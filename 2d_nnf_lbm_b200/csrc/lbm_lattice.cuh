@@ -1419,6 +1419,9 @@ __device__ __forceinline__ void node_force(const LatticeArgs& a, const Cand& C,
     if (parked) {
 #pragma unroll
       for (int k = 0; k < 9; ++k) f[k] = q[ST::off(k)];
+      // the stage was written by ordinary stores and is refilled by TMA: the
+      // warp's arrival on "empty" orders the two only behind this fence
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
   }
   v.rho = rho;
