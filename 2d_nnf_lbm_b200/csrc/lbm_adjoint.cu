@@ -847,7 +847,7 @@ __global__ void __launch_bounds__(LEVELS_TPB, 1) k_adj_levels(const AdjLevelsArg
   };
   const uint32_t force_bar = (uint32_t)__cvta_generic_to_shared(&s_force);
   if (tid == 0) {
-    s_stop = 0;
+    s_stop = timed_out(a.status) ? 1 : 0;
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(force_bar) : "memory");
   }
   if (disk) {
@@ -859,6 +859,7 @@ __global__ void __launch_bounds__(LEVELS_TPB, 1) k_adj_levels(const AdjLevelsArg
     load_disk(a.n_hi);
   }
   __syncthreads();
+  if (s_stop) return;
   double gnu = 0.0, gty = 0.0;
   // the forward half of one segment at level n
   int i = 0, j = 0;

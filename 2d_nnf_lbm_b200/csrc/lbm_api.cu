@@ -923,25 +923,10 @@ bool steps_resident(const lbm_sim* h) {
          nodes(h) + STEPS_NODES_PER_DISK * h->np <= STEPS_MAX_NODES;
 }
 
-// Up to `left` time steps in one launch on the handle's stream; *done: how
-// many (bounded by the room in the history ring).
-// slots: the populations and omega are read from the 10-plane block there and
-// written to the blocks after it, one per step (the handle's own stay).
-int enqueue_steps(lbm_sim* h, int left, int* done, unsigned char* slots = nullptr) {
-  const int every = h->p.series_every;
-  int n = std::min(left, STEPS_MAX_LAUNCH);
-  if (h->series && every > 0) {
-    if ((h->kk + 1) / every - h->copied_kk / every > h->series_cap) {
-      int rc = series_enqueue(h);  // the ring slots are copied before reuse
-      if (rc) return rc;
-    }
-    const long long last = (h->copied_kk / every + h->series_cap + 1) * (long long)every - 1;
-    n = (int)std::min<long long>(n, last - h->kk);
-    if ((h->kk + n) / every > h->kk / every) {
-      int rc = ring_wait(h, (h->kk + n) / every - 1);
-      if (rc) return rc;
-    }
-  }
+// Arguments of a launch of k_steps over the next n steps.  slots: the
+// populations and omega are read from the 10-plane block there and written to
+// the blocks after it, one per step (the handle's own stay).
+StepsArgs steps_args(lbm_sim* h, int n, unsigned char* slots) {
   StepsArgs q{};
   if (slots) {
     const size_t pb = (size_t)h->g.plane * h->esz;
@@ -967,10 +952,31 @@ int enqueue_steps(lbm_sim* h, int left, int* done, unsigned char* slots = nullpt
   q.kk0 = h->kk;
   q.nsteps = n;
   q.decode0 = h->partials_valid ? 1 : 0;
+  q.bar0 = h->steps_bar_base;
+  return q;
+}
+
+// Up to `left` time steps in one launch on the handle's stream; *done: how
+// many (bounded by the room in the history ring).  slots: see steps_args.
+int enqueue_steps(lbm_sim* h, int left, int* done, unsigned char* slots = nullptr) {
+  const int every = h->p.series_every;
+  int n = std::min(left, STEPS_MAX_LAUNCH);
+  if (h->series && every > 0) {
+    if ((h->kk + 1) / every - h->copied_kk / every > h->series_cap) {
+      int rc = series_enqueue(h);  // the ring slots are copied before reuse
+      if (rc) return rc;
+    }
+    const long long last = (h->copied_kk / every + h->series_cap + 1) * (long long)every - 1;
+    n = (int)std::min<long long>(n, last - h->kk);
+    if ((h->kk + n) / every > h->kk / every) {
+      int rc = ring_wait(h, (h->kk + n) / every - 1);
+      if (rc) return rc;
+    }
+  }
+  const StepsArgs q = steps_args(h, n, slots);
   const LatticeArgs a = lattice_args(h);
   const ParticleArgs pa = particle_args(h);
   int grid = 0;
-  q.bar0 = h->steps_bar_base;
   CK(h->prec == LBM_FP64 ? launch_steps_fp64(a, pa, q, h->stream, &grid)
                          : launch_steps_fp32(a, pa, q, h->stream, &grid));
   h->steps_bar_base += (unsigned)(n - 1) * (unsigned)grid;
@@ -1622,9 +1628,20 @@ int lbm_get_status(lbm_sim* h) {
 int lbm_selftest_wait(lbm_sim* h, int32_t limit) {
   if (!h || limit < 1 || limit > (1 << 20)) return LBM_E_INVALID;
   cudaSetDevice(h->p.device);
-  CK(launch_wait_selftest(h->d_status, (uint32_t)limit, h->stream));
+  CK(launch_wait_selftest(h->steps_bar, h->steps_bar_base + 1, h->d_status, (uint32_t)limit,
+                          h->stream));
+  long long kk = h->kk;
+  if (steps_resident(h)) {
+    const LatticeArgs a = lattice_args(h);
+    const ParticleArgs pa = particle_args(h);
+    const StepsArgs q = steps_args(h, 2, nullptr);
+    int grid = 0;
+    CK(h->prec == LBM_FP64 ? launch_steps_fp64(a, pa, q, h->stream, &grid)
+                           : launch_steps_fp32(a, pa, q, h->stream, &grid));
+    CK(d2h(h, &kk, h->d_kk, sizeof(kk)));
+  }
   CK(d2h(h, h->h_status, h->d_status, sizeof(int)));
-  return LBM_OK;
+  return kk == h->kk ? LBM_OK : LBM_E_STATE;
 }
 
 int32_t lbm_checked_build(void) {

@@ -319,7 +319,8 @@ cudaError_t launch_batch_tma_fp64(const BatchSim* sims, int nsim, const CUtensor
 cudaError_t batch_tma_prepare_fp32(int stress, int* blocks_per_sm);
 cudaError_t batch_tma_prepare_fp64(int stress, int* blocks_per_sm);
 cudaError_t prepare_particles_batch();
-cudaError_t launch_wait_selftest(int* status, uint32_t limit, cudaStream_t s);
+cudaError_t launch_wait_selftest(const unsigned* grid_bar, unsigned target, int* status,
+                                 uint32_t limit, cudaStream_t s);
 cudaError_t launch_particles_batch(const ParticleArgs* args, int nsim, cudaStream_t s);
 
 // ---------------------------------------------------------------------------

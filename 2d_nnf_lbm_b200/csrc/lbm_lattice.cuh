@@ -48,14 +48,25 @@ __device__ __forceinline__ void grid_arrive(unsigned* bar) {
   asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
 }
 // False if it did not complete within the limit.
-__device__ __forceinline__ bool grid_wait(const unsigned* bar, unsigned target, int* status) {
-  for (int it = 0; it < (1 << 22); ++it) {
+__device__ __forceinline__ bool grid_poll(const unsigned* bar, unsigned target, uint32_t limit) {
+  for (uint32_t it = 0; it < limit; ++it) {
     unsigned v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
     if ((int)(v - target) >= 0) return true;
   }
+  return false;
+}
+__device__ __forceinline__ bool grid_wait(const unsigned* bar, unsigned target, int* status) {
+  if (grid_poll(bar, target, 1u << 22)) return true;
   atomicOr(status, ST_TIMEOUT);
   return false;
+}
+// Whether a wait of an earlier launch expired.  The host counts each launch's
+// arrivals when it queues it, so behind an expired grid barrier the count
+// stays short and every later launch would poll its limit out as well
+// (seconds each): a kernel with a grid barrier returns at once instead.
+__device__ __forceinline__ bool timed_out(const int* status) {
+  return (*static_cast<const volatile int*>(status) & ST_TIMEOUT) != 0;
 }
 
 // A load of data that other blocks write during the launch (CG: past the L1

@@ -277,16 +277,19 @@ __global__ void __launch_bounds__(STEPS_TPB, 1)
     if (f == P_X || f == P_Y) S.pos[q.kk0 & 1][f == P_X ? 0 : 1][id] = v;
   }
   if (tid == 0) {
-    S.stop = S.moved = S.n = 0;
+    S.stop = timed_out(a.status) ? 1 : 0;
+    S.moved = S.n = 0;
     S.next = S.next_late = S.n_late = 0;
     S.mass = 0ull;
     S.stale = __ldcg(q.stale + q.stale0);
   }
   __syncthreads();
+  const int nsteps = S.stop ? 0 : q.nsteps;
   if (p.np > 0) steps_lists(p, S, (int)(q.kk0 & 1), row0, row1);
   const bool disk_warp = warp * 32 < p.np;
   if (disk_warp) steps_disk_terms(p, S, q.kk0 + 1);
-  for (int s = 1; s <= q.nsteps; ++s) {
+  int done = 0;
+  for (int s = 1; s <= nsteps; ++s) {
     const long long kk = q.kk0 + s;
     const bool rec = p.series != nullptr && p.series_every > 0 && kk % p.series_every == 0;
     const long long from = (s - 1) & q.mask, to = s & q.mask;
@@ -387,7 +390,8 @@ __global__ void __launch_bounds__(STEPS_TPB, 1)
     // ---- to the next step: the last warp keeps the barrier, the first ones
     //      prepare the disks meanwhile
     __syncthreads();
-    if (s == q.nsteps) break;
+    done = s;
+    if (s == nsteps) break;
     if (tid == STEPS_TPB - 32) {
       S.next = S.next_late = S.n_late = 0;
       grid_arrive(q.bar);
@@ -395,12 +399,13 @@ __global__ void __launch_bounds__(STEPS_TPB, 1)
     }
     if (disk_warp) steps_disk_terms(p, S, kk + 1);
     __syncthreads();
-    if (S.stop) return;
+    if (S.stop) break;
   }
-  // ---- the state of step kk0 + nsteps, into the other copy (a block that
-  //      starts late may still be reading the first) -------------------------
+  // ---- the state of the last step, into the other copy (a block that starts
+  //      late may still be reading the first); after an expired wait too, as
+  //      the host goes on with that copy ---------------------------------------
   if (blockIdx.x == 0) {
-    const long long kk = q.kk0 + q.nsteps;
+    const long long kk = q.kk0 + done;
     for (int e = tid; e < PS * p.np; e += STEPS_TPB) {
       const int f = e / p.np, id = e - f * p.np;
       const double v = f == P_X || f == P_Y ? S.pos[kk & 1][f == P_X ? 0 : 1][id] : S.rec[f][id];

@@ -256,11 +256,14 @@ int lbm_get_status(lbm_sim* h);
 
 /* Check of the failure path of the kernels' bounded waits (no counterpart in
  * the reference): on the handle's stream, one thread waits on a fresh
- * mbarrier that nothing arrives at, with the same bounded wait the step
- * kernel uses, and gives up after `limit` polls (1..1048576), setting the
- * handle's timeout status as a step kernel whose wait expired does.  The
- * handle then reports LBM_E_TIMEOUT from lbm_get_status and refuses further
- * steps (sticky); the device and other handles are unaffected. */
+ * mbarrier that nothing arrives at and for a grid barrier count that never
+ * comes, with the same bounded waits the kernels use, and gives each up after
+ * `limit` polls (1..1048576), setting the handle's timeout status as a kernel
+ * whose wait expired does.  Where the handle steps many steps per launch, such
+ * a launch is queued behind it, as a long lbm_step may have done: it has to
+ * return without a step (else LBM_E_STATE).  The handle then reports
+ * LBM_E_TIMEOUT from lbm_get_status and refuses further steps (sticky); the
+ * device and other handles are unaffected. */
 int lbm_selftest_wait(lbm_sim* h, int32_t limit);
 
 /* The handle's CUDA stream (a cudaStream_t), so a caller can order its own
