@@ -60,6 +60,7 @@ struct lbm_sim {
   unsigned long long* facc = nullptr;  // [6][npad] FORCE accumulators in use, one of
   unsigned long long* facc3 = nullptr;  // [3][6][npad] (k_steps rotates them)
   bool lists_stale = false;  // k_steps moved the disks: the tile and pair lists are old
+  int steps_grid = 0;                  // blocks of k_steps on this lattice, 0: it does not fit
   unsigned* steps_bar = nullptr;       // k_steps' grid barrier
   unsigned steps_bar_base = 0;         // its count so far
   int* rec_slot = nullptr;
@@ -918,8 +919,10 @@ int enqueue_step(lbm_sim* h) {
 // TMA tiles) and with the disks (each block updates all of them): at 513 x 513
 // with 100 disks 14.5 / 14.7 (FP64) and 12.4 / 13.0, with 200 disks 17.8 / 16.4
 // and 15.1 / 14.4.
+// A lattice with more row segments than k_steps' queues hold (steps_grid 0)
+// takes the two kernels at any node count.
 bool steps_resident(const lbm_sim* h) {
-  return !h->prof && !h->m.bgk && h->np <= STEPS_MAX_DISKS &&
+  return h->steps_grid > 0 && !h->prof && !h->m.bgk && h->np <= STEPS_MAX_DISKS &&
          nodes(h) + STEPS_NODES_PER_DISK * h->np <= STEPS_MAX_NODES;
 }
 
@@ -976,10 +979,9 @@ int enqueue_steps(lbm_sim* h, int left, int* done, unsigned char* slots = nullpt
   const StepsArgs q = steps_args(h, n, slots);
   const LatticeArgs a = lattice_args(h);
   const ParticleArgs pa = particle_args(h);
-  int grid = 0;
-  CK(h->prec == LBM_FP64 ? launch_steps_fp64(a, pa, q, h->stream, &grid)
-                         : launch_steps_fp32(a, pa, q, h->stream, &grid));
-  h->steps_bar_base += (unsigned)(n - 1) * (unsigned)grid;
+  CK(h->prec == LBM_FP64 ? launch_steps_fp64(a, pa, q, h->stream, h->steps_grid)
+                         : launch_steps_fp32(a, pa, q, h->stream, h->steps_grid));
+  h->steps_bar_base += (unsigned)(n - 1) * (unsigned)h->steps_grid;
   h->kk += n;
   if (!slots) h->cur ^= n & 1;
   std::swap(h->ps, h->ps_alt);
@@ -1189,6 +1191,10 @@ int lbm_create(const lbm_params* pin, lbm_sim** out) {
       cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&h->copy_fork, cudaEventDisableTiming) != cudaSuccess)
     return fail(LBM_E_CUDA);
+  int sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.device) != cudaSuccess)
+    return fail(LBM_E_CUDA);
+  h->steps_grid = steps_grid(h->g, sms);
   const size_t pin0 = (size_t)32 * (PS + 6);  // ps_pin for up to 32 disks
   if (cudaHostAlloc(reinterpret_cast<void**>(&h->status_pin),
                     STATUS_PIN_HEAD + pin0 * sizeof(double), cudaHostAllocDefault) != cudaSuccess)
@@ -1635,9 +1641,8 @@ int lbm_selftest_wait(lbm_sim* h, int32_t limit) {
     const LatticeArgs a = lattice_args(h);
     const ParticleArgs pa = particle_args(h);
     const StepsArgs q = steps_args(h, 2, nullptr);
-    int grid = 0;
-    CK(h->prec == LBM_FP64 ? launch_steps_fp64(a, pa, q, h->stream, &grid)
-                           : launch_steps_fp32(a, pa, q, h->stream, &grid));
+    CK(h->prec == LBM_FP64 ? launch_steps_fp64(a, pa, q, h->stream, h->steps_grid)
+                           : launch_steps_fp32(a, pa, q, h->stream, h->steps_grid));
     CK(d2h(h, &kk, h->d_kk, sizeof(kk)));
   }
   CK(d2h(h, h->h_status, h->d_status, sizeof(int)));

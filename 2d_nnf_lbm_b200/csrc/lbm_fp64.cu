@@ -35,7 +35,7 @@ cudaError_t launch_bgk_step_fp64(const LatticeArgs& a, cudaStream_t s) {
   return launch_mode<double>(a, s, MODE_STEP);
 }
 cudaError_t launch_steps_fp64(const LatticeArgs& a, const ParticleArgs& p, const StepsArgs& q,
-                              cudaStream_t s, int* grid) {
+                              cudaStream_t s, int grid) {
   return launch_steps<double>(a, p, q, s, grid);
 }
 }  // namespace lbm

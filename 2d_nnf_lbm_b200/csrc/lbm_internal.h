@@ -212,9 +212,27 @@ struct LatticeArgs {
 };
 
 // Several time steps of a small simulation in one launch (lbm_steps.cuh);
-// launch_steps_* set *grid to the blocks launched, each of which arrives at
-// the barrier nsteps - 1 times.
+// each of the grid blocks arrives at the barrier nsteps - 1 times.
 constexpr int STEPS_MAX_DISKS = 256;
+// 32-node row segments a block has at least, on a lattice with fewer than one
+// for every warp of the chip: the warps then share their SM with fewer others.
+// FP64 us per step with 16 / 12 / 8 / 4: 81 x 301 Bingham 7.80 / 7.65 / 7.53 /
+// 7.50, 101 x 301 5.98 / 5.77 / 5.65 / 5.64, 161 x 161 with 8 disks 7.06 / 6.82 /
+// 6.66 / 6.65.
+constexpr int STEPS_MIN_SEGS = 8;
+constexpr int STEPS_MAX_SEGS = 512;  // and at most (the block's queue)
+// A row takes a segment however narrow the lattice is.
+inline long long steps_segments(const Geometry& g) {
+  return (long long)((g.nx + 32) / 32) * (g.ny + 1);
+}
+// Blocks of a launch on a GPU of sms SMs, 0 if the lattice has more segments
+// than their queues hold (on 148 SMs: rows of one segment, above 75,776 rows).
+inline int steps_grid(const Geometry& g, int sms) {
+  const long long n = steps_segments(g);
+  const long long want = (n + STEPS_MIN_SEGS - 1) / STEPS_MIN_SEGS;
+  const int grid = (int)(want < sms ? want : sms);
+  return grid > 0 && (n + grid - 1) / grid <= STEPS_MAX_SEGS ? grid : 0;
+}
 struct StepsArgs {
   // step s (1..nsteps) reads the populations at f + ((s-1) & mask) * f_stride
   // (bytes) and writes those at f + (s & mask) * f_stride; omega likewise.
@@ -235,9 +253,9 @@ struct StepsArgs {
   int decode0;               // the accumulators hold FORCE of step kk0
 };
 cudaError_t launch_steps_fp64(const LatticeArgs& a, const ParticleArgs& p, const StepsArgs& q,
-                              cudaStream_t s, int* grid);
+                              cudaStream_t s, int grid);
 cudaError_t launch_steps_fp32(const LatticeArgs& a, const ParticleArgs& p, const StepsArgs& q,
-                              cudaStream_t s, int* grid);
+                              cudaStream_t s, int grid);
 
 // Launchers (defined in lbm_fp64.cu / lbm_fp32.cu).
 cudaError_t launch_init_fp64(const LatticeArgs& a, cudaStream_t s);

@@ -34,13 +34,6 @@ namespace lbm {
 
 constexpr int STEPS_TPB = 512;
 constexpr int STEPS_WARPS = STEPS_TPB / 32;
-// Segments a block has at least, on a lattice with fewer than one for every
-// warp of the chip: the warps then share their SM with fewer others.  FP64 us
-// per step with 16 / 12 / 8 / 4: 81 x 301 Bingham 7.80 / 7.65 / 7.53 / 7.50,
-// 101 x 301 5.98 / 5.77 / 5.65 / 5.64, 161 x 161 with 8 disks 7.06 / 6.82 /
-// 6.66 / 6.65.
-constexpr int STEPS_MIN_SEGS = 8;
-constexpr int STEPS_MAX_SEGS = 512;  // segments of a block
 
 struct StepsShared {
   double rec[PS][STEPS_MAX_DISKS];     // disk records (P_X, P_Y: pos instead)
@@ -420,23 +413,13 @@ __global__ void __launch_bounds__(STEPS_TPB, 1)
 
 template <class T>
 cudaError_t launch_steps(const LatticeArgs& a, const ParticleArgs& p, const StepsArgs& q,
-                         cudaStream_t s, int* grid_out) {
+                         cudaStream_t s, int grid) {
   const int sx = (a.m.bingham || a.m.record_stress) ? 1 : 0;
   void (*const kern)(const LatticeArgs, const ParticleArgs, const StepsArgs) =
       sx ? k_steps<T, true> : k_steps<T, false>;
-  int dev = 0, sms = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(StepsShared));
   if (e != cudaSuccess) return e;
-  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
-    return e;
-  if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(StepsShared))) != cudaSuccess)
-    return e;
-  const long long nseg = (long long)((a.g.nx + 32) / 32) * (a.g.ny + 1);
-  const int want = (int)((nseg + STEPS_MIN_SEGS - 1) / STEPS_MIN_SEGS);
-  const int grid = want < sms ? want : sms;
-  *grid_out = grid;
-  if ((nseg + grid - 1) / grid > STEPS_MAX_SEGS) return cudaErrorInvalidValue;
   LatticeArgs la = a;
   ParticleArgs pa = p;
   StepsArgs qa = q;
