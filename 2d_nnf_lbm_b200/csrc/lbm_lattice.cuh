@@ -218,6 +218,22 @@ __device__ __forceinline__ float phi_float(float di, float dj, float R, float ze
   return phi;
 }
 
+// Velocity at (di, dj) from the centre of a disk that moves with (u, v, w):
+// FP64 in the reference's arithmetic (C1:488-542), FP32 fused.  Every kernel
+// that evaluates it takes it from here, so single, resident and batched runs
+// (either batch kernel: the autotuner chooses by time) round alike.
+template <class T>
+__device__ __forceinline__ void rigid_velocity(double u, double v, double w, double di, double dj,
+                                               T& ux, T& uy) {
+  if (sizeof(T) == 8) {
+    ux = (T)u - (T)w * (T)dj;
+    uy = (T)v + (T)w * (T)di;
+  } else {
+    ux = fmaf(-(float)w, (float)dj, (float)u);
+    uy = fmaf((float)w, (float)di, (float)v);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Stress, yield code and omega a collision leaves for the next one.
 struct NodeOut {
@@ -837,8 +853,8 @@ __device__ __forceinline__ void lattice_body(const LatticeArgs& a, int bxi, int 
         phi = (T)phi_float((float)di, (float)dj, (float)s_pr[c], m.zeta_f, m.pi_f);
       if (phi > (T)0) {
         hit = true;
-        const T uxp = (T)s_pu[c] - (T)s_pw[c] * (T)dj;
-        const T uyp = (T)s_pv[c] + (T)s_pw[c] * (T)di;
+        T uxp, uyp;
+        rigid_velocity<T>(s_pu[c], s_pv[c], s_pw[c], di, dj, uxp, uyp);
         if (!initial) {
           gx = phi * (uxp - ux);
           gy = phi * (uyp - uy);
@@ -1386,13 +1402,7 @@ __device__ __forceinline__ void node_force(const LatticeArgs& a, const Cand& C,
         if (phi > (T)0) {
           hit = true;
           T uxp, uyp;
-          if (F64) {
-            uxp = (T)C.u(c) - (T)C.w(c) * (T)dj;
-            uyp = (T)C.v(c) + (T)C.w(c) * (T)di;
-          } else {
-            uxp = fmaf(-(float)C.w(c), (float)dj, (float)C.u(c));
-            uyp = fmaf((float)C.w(c), (float)di, (float)C.v(c));
-          }
+          rigid_velocity<T>(C.u(c), C.v(c), C.w(c), di, dj, uxp, uyp);
           if (C.id(c) > gbest) {
             gbest = C.id(c);
             gx = phi * (uxp - ux);
