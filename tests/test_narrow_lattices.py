@@ -46,11 +46,11 @@ def test_narrow_lattice_steps(pkg, cases, nx, ny, precision):
 def test_narrow_lattice_adjoint(pkg, cases):
     """lbm_adjoint above the line: the gradient of the one-launch-per-kernel
     path (the same kernels; its sums are atomics, 1e-9 as in test_adjoint)."""
-    p = cases.shipped_c1(4, 79990, 2.0)
+    p = cases.shipped_c1(3, 80000, 2.0)
     p.gravity = -1e-5
     p.wall_model = 2
     p.series_every = 0
-    pin = cases.pin_array([[2.1, 40000.2]], 2.0, 1.25)
+    pin = cases.pin_array([[1.6, 40000.2]], 1.0, 1.25)
     out = []
     for profiled in (False, True):
         s = pkg.Simulation(p)
