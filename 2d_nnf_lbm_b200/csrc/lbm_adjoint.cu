@@ -881,7 +881,8 @@ __global__ void __launch_bounds__(LEVELS_TPB, 1) k_adj_levels(const AdjLevelsArg
     j = seg / spr;
     const int i0 = (seg - j * spr) * 32;
     i = i0 + lane;
-    act = i <= g.nx;
+    act = i <= g.nx && LBM_IN(i0, g.nx + 1, a.status) && LBM_IN(j, g.ny + 1, a.status) &&
+          LBM_IN(n - a.n_lo, a.n_hi - a.n_lo + 1, a.status);
     T h[9];
     adj_load_fwd<T>(g, m, io, i, j, act, h, om);
 #pragma unroll

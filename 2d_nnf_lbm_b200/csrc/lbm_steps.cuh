@@ -98,7 +98,8 @@ static __device__ __noinline__ void steps_lists(const ParticleArgs& p, StepsShar
     if (w < warp) before += S.wcount[w];
     total += S.wcount[w];
   }
-  if (need) S.idx[before + __popc(m & ((1u << lane) - 1))] = tid;
+  const int pos = before + __popc(m & ((1u << lane) - 1));
+  if (need && LBM_IN(pos, STEPS_MAX_DISKS, p.status)) S.idx[pos] = tid;
   if (tid == 0) S.n = total;
   __syncthreads();
 }
@@ -118,9 +119,11 @@ __device__ __forceinline__ void steps_disk_terms(const ParticleArgs& p, StepsSha
 #pragma unroll
       for (int iw = 1; iw <= 4; ++iw) D_PW = wall_force(p, iw, px, py, pd, wf[iw - 1]);
     }
-    const int nn = S.nn[id];
+    int nn = S.nn[id];
+    if (!LBM_IN(nn, MAX_NEIGH + 1, p.status)) nn = 0;
     for (int k = 0; k < nn; ++k) {  // pairs, then walls 1 to 4: the reference's order
       const int o = S.nbr[k][id];
+      if (!LBM_IN(o, p.np, p.status)) continue;
       const double ox = X[o], oy = Y[o], od = S.rec[P_D][o];
       if (!pair_near(px, py, pd, ox, oy, od, p.rep_zeta)) continue;
       double F[2];
@@ -231,13 +234,16 @@ __device__ __forceinline__ void steps_disk_update(const ParticleArgs& p, const S
     atomicOr(p.status, ST_PARTICLE);
   if (p.series != nullptr && p.series_every > 0 && kk % p.series_every == 0 && id < p.series_np) {
     const long long slot = (kk / p.series_every - 1) % p.series_cap;
-    double* r = p.series + slot * p.series_len + 2 + 12LL * id;
-    r[0] = d.x; r[1] = d.y; r[2] = d.ang;
-    r[3] = d.u; r[4] = d.v; r[5] = d.w;
-    r[6] = d.fx; r[7] = d.fy; r[8] = d.tz;
-    r[9] = S.rec[P_FHX][id]; r[10] = S.rec[P_FHY][id]; r[11] = S.rec[P_FHT][id];
+    const long long off = slot * p.series_len + 2 + 12LL * id;
+    if (LBM_IN(off + 11, (long long)p.series_cap * p.series_len, p.status)) {
+      double* r = p.series + off;
+      r[0] = d.x; r[1] = d.y; r[2] = d.ang;
+      r[3] = d.u; r[4] = d.v; r[5] = d.w;
+      r[6] = d.fx; r[7] = d.fy; r[8] = d.tz;
+      r[9] = S.rec[P_FHX][id]; r[10] = S.rec[P_FHY][id]; r[11] = S.rec[P_FHT][id];
+    }
   }
-  if (p.hist && kk < p.hist_n) {
+  if (p.hist && kk < p.hist_n && LBM_IN(kk, p.hist_n, p.status)) {
     double* h = p.hist + kk * (long long)PS * st + id;
     for (int f = 2; f < PS; ++f) h[(long long)f * st] = S.rec[f][id];
     h[P_X * (long long)st] = d.x;
@@ -295,6 +301,9 @@ __global__ void __launch_bounds__(STEPS_TPB, 1)
     // one segment of 32 nodes; nc listed disks at the centres of step kk
     auto segment = [&](int seg, int nc) {
       const int j = row_of(seg), i0 = (seg - j * spr) * 32, i = i0 + lane;
+      if (!LBM_IN(seg - seg0, seg1 - seg0, a.status) || !LBM_IN(j, g.ny + 1, a.status) ||
+          !LBM_IN(i0, g.nx + 1, a.status))
+        return;
       const bool act = i <= g.nx;
       const long long nd = (long long)j * g.pitch + i;
       NodeVals<T> v;
@@ -328,8 +337,8 @@ __global__ void __launch_bounds__(STEPS_TPB, 1)
       const int j = row_of(seg), i0 = (seg - j * spr) * 32;
       for (int c0 = 0; c0 < S.n; c0 += 32) {
         bool nr = false;
-        if (c0 + lane < S.n) {
-          const int id = S.idx[c0 + lane];
+        const int id = c0 + lane < S.n ? S.idx[c0 + lane] : -1;
+        if (id >= 0 && LBM_IN(id, p.np, a.status)) {
           const double dl = (double)i0 - X[id], dr = dl + 31.0;
           const double dx = dl > 0.0 ? dl : (dr < 0.0 ? -dr : 0.0), dy = (double)j - Y[id];
           const double reach = 0.5 * S.rec[P_D][id] + 0.5 * m.zeta + 1.0 + SKIN;
@@ -352,7 +361,10 @@ __global__ void __launch_bounds__(STEPS_TPB, 1)
     }
     for (int e; (e = take(&S.next, seg1 - seg0)) >= 0;) {
       if (S.n > 0 && may_reach(seg0 + e)) {
-        if (lane == 0) S.late[atomicAdd(&S.n_late, 1)] = seg0 + e;
+        if (lane == 0) {
+          const int w = atomicAdd(&S.n_late, 1);
+          if (LBM_IN(w, STEPS_MAX_SEGS, a.status)) S.late[w] = seg0 + e;
+        }
       } else {
         segment(seg0 + e, 0);
       }
@@ -372,9 +384,10 @@ __global__ void __launch_bounds__(STEPS_TPB, 1)
       __syncthreads();
       if (tid == 0) {
         const long long slot = (kk / p.series_every - 1) % p.series_cap;
-        if (S.mass) atomicAdd(p.mass_acc + slot, S.mass);
+        const bool in = LBM_IN(slot, p.series_cap, a.status);
+        if (S.mass && in) atomicAdd(p.mass_acc + slot, S.mass);
         S.mass = 0ull;
-        if (blockIdx.x == 0) {
+        if (blockIdx.x == 0 && in) {
           p.series[slot * p.series_len + 0] = (double)kk;
           p.series[slot * p.series_len + 1] = __longlong_as_double(0x7ff8000000000000LL);
         }
