@@ -12,12 +12,16 @@
 // kernel re-derives the fields of step K (F after BC, rho, u, G, PHI) on
 // demand without touching the state.
 #include <algorithm>
+#include <chrono>
+#include <climits>
 #include <cmath>
 #include <deque>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <new>
+#include <thread>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -63,6 +67,10 @@ struct lbm_sim {
   int steps_grid = 0;                  // blocks of k_steps on this lattice, 0: it does not fit
   unsigned* steps_bar = nullptr;       // k_steps' grid barrier
   unsigned steps_bar_base = 0;         // its count so far
+  int sms = 0;                         // SMs of the device
+  // while the handle is among the running ones (start_running; their mutex)
+  long long run_until = 0;             // idle once h_kk shows this step
+  int run_claim = 0;                   // SMs its launches occupy
   int* rec_slot = nullptr;
   int* tile_count = nullptr;
   int* tile_list = nullptr;
@@ -85,10 +93,11 @@ struct lbm_sim {
   double cell_size = 1.0;
   // scalars
   unsigned long long* mass_acc = nullptr;
-  long long* d_kk = nullptr;
+  long long* d_kk = nullptr;  // steps done; d_status follows it
   double* stale_dpw = nullptr;   // D_PW in use, one of
   double* stale_dpw2 = nullptr;  // [2] (k_steps alternates them)
-  unsigned char* status_pin = nullptr;  // pinned: h_status, then ps_pin's first home
+  unsigned char* status_pin = nullptr;  // pinned: h_kk, h_status, then ps_pin's first home
+  long long* h_kk = nullptr;  // pinned copy of d_kk as of the last completed lbm_step
   int* h_status = nullptr;  // pinned copy of d_status, refreshed after each call
   int* d_status = nullptr;  // sticky ST_* bits written by the kernels
   // history
@@ -157,6 +166,7 @@ namespace {
 constexpr int NOUT = 7;  // ux uy rho phi gx gy pnode
 constexpr size_t STATUS_PIN_HEAD = 64;  // bytes of status_pin before ps_pin
 constexpr int STEPS_MAX_LAUNCH = 1024;  // time steps per launch of k_steps
+constexpr int STEPS_RECHECK = 256;      // steps between two looks at the other handles
 #ifndef LBM_STEPS_MAX_NODES
 #define LBM_STEPS_MAX_NODES 400000
 #endif
@@ -247,6 +257,60 @@ int refreshed_status(lbm_sim* h) {
     return LBM_E_CUDA;
   return sticky_status(h);
 }
+
+// The handles of this process whose steps may still run.  A launch of k_steps
+// holds its SMs for milliseconds (no second block fits one), so two handles
+// stepping at once would take turns where the particle and step kernels overlap
+// their latencies: 2 / 4 threads with a handle each, us per step of one handle,
+// k_steps / two kernels, FP64: 101 x 301 6.0 / 5.0 and 6.0 / 2.8, 201 x 601 7.2 /
+// 5.4 and 7.2 / 5.0, 81 x 301 Bingham 8.7 / 6.4 and 8.7 / 3.5 (alone 6.0 / 8.8,
+// 7.3 / 9.8, 8.8 / 11.9); 32 x 64, where a launch takes 17 SMs and several run at
+// once, 2.9 / 4.8 and 1.5 / 2.7.  So a handle takes the resident kernels only
+// while its blocks and those of the other running handles find an SM each.  It
+// reads the pinned step counters that lbm_step has copied back, no CUDA call.
+struct Running {
+  std::mutex mu;
+  std::vector<lbm_sim*> sims;
+};
+Running& running() {
+  static Running* r = new Running;  // handles may outlive static destructors
+  return *r;
+}
+
+// Notes that h occupies `claim` SMs until its step counter shows `until`
+// (LLONG_MAX: until stop_running); whether all that runs then fits the device.
+bool start_running(lbm_sim* h, long long until, int claim) {
+  Running& r = running();
+  std::lock_guard<std::mutex> lock(r.mu);
+  long long used = claim;
+  size_t n = 0;
+  for (lbm_sim* q : r.sims) {
+    const bool idle = *(volatile long long*)q->h_kk == q->run_until ||
+                      *(volatile int*)q->h_status != 0;  // a failed handle steps no more
+    if (q == h || idle) continue;
+    r.sims[n++] = q;
+    if (q->p.device == h->p.device) used += q->run_claim;
+  }
+  r.sims.resize(n);
+  r.sims.push_back(h);
+  h->run_until = until;
+  h->run_claim = claim;
+  return used <= h->sms;
+}
+
+void stop_running(lbm_sim* h) {
+  Running& r = running();
+  std::lock_guard<std::mutex> lock(r.mu);
+  r.sims.erase(std::remove(r.sims.begin(), r.sims.end(), h), r.sims.end());
+}
+
+// The same for the length of a call that returns when its work is done.
+struct RunningScope {
+  lbm_sim* h;
+  bool room;
+  RunningScope(lbm_sim* h_, int claim) : h(h_), room(start_running(h_, LLONG_MAX, claim)) {}
+  ~RunningScope() { stop_running(h); }
+};
 
 LatticeArgs lattice_args(lbm_sim* h) {
   LatticeArgs a{};
@@ -817,6 +881,7 @@ int make_tensor_maps(lbm_sim* h) {
 }
 
 void destroy_buffers(lbm_sim* h) {
+  stop_running(h);
   // history copies still in flight on the copy stream read the device ring
   // and write the pinned staging ring: let them finish before anything goes
   if (h->copy_stream) cudaStreamSynchronize(h->copy_stream);
@@ -991,6 +1056,31 @@ int enqueue_steps(lbm_sim* h, int left, int* done, unsigned char* slots = nullpt
   h->partials_valid = true;
   h->lists_stale = true;
   *done = n;
+  return LBM_OK;
+}
+
+// The step counter and the status to the host, behind the steps queued so far.
+int copy_progress(lbm_sim* h) {
+  CK(cudaMemcpyAsync(h->h_kk, h->d_kk, 2 * sizeof(long long), cudaMemcpyDeviceToHost, h->stream));
+  return LBM_OK;
+}
+
+// Between two launches of k_steps in one call: waits until no more than one
+// launch's steps are still to run, so that a call of many steps can give way to
+// a handle that starts meanwhile (the launches of the two kernels hold their
+// caller back in the same way, by the depth of the launch queue).
+int steps_throttle(lbm_sim* h) {
+  int rc = copy_progress(h);
+  if (rc) return rc;
+  const auto t0 = std::chrono::steady_clock::now();
+  while (*(volatile long long*)h->h_kk < h->kk - STEPS_MAX_LAUNCH &&
+         *(volatile int*)h->h_status == 0) {
+    if (std::chrono::steady_clock::now() - t0 > std::chrono::seconds(1)) {
+      CK(cudaStreamSynchronize(h->stream));  // or the error that keeps the copy away
+      break;
+    }
+    std::this_thread::sleep_for(std::chrono::microseconds(50));
+  }
   return LBM_OK;
 }
 
@@ -1191,15 +1281,16 @@ int lbm_create(const lbm_params* pin, lbm_sim** out) {
       cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&h->copy_fork, cudaEventDisableTiming) != cudaSuccess)
     return fail(LBM_E_CUDA);
-  int sms = 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.device) != cudaSuccess)
+  if (cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, p.device) != cudaSuccess)
     return fail(LBM_E_CUDA);
-  h->steps_grid = steps_grid(h->g, sms);
+  h->steps_grid = steps_grid(h->g, h->sms);
   const size_t pin0 = (size_t)32 * (PS + 6);  // ps_pin for up to 32 disks
   if (cudaHostAlloc(reinterpret_cast<void**>(&h->status_pin),
                     STATUS_PIN_HEAD + pin0 * sizeof(double), cudaHostAllocDefault) != cudaSuccess)
     return fail(LBM_E_NOMEM);
-  h->h_status = reinterpret_cast<int*>(h->status_pin);
+  h->h_kk = reinterpret_cast<long long*>(h->status_pin);
+  h->h_status = reinterpret_cast<int*>(h->h_kk + 1);
+  *h->h_kk = 0;
   h->ps_pin = reinterpret_cast<double*>(h->status_pin + STATUS_PIN_HEAD);
   h->ps_pin_n = pin0;
   *h->h_status = 0;
@@ -1226,15 +1317,15 @@ int lbm_create(const lbm_params* pin, lbm_sim** out) {
     b.add(&h->work_ctr, 2);
     b.add(&h->pair_rebuild, 1);
     b.add(&h->rec_slot, 1);
-    b.add(&h->d_kk, 1);
+    b.add(&h->d_kk, 2);
     b.add(&h->stale_dpw2, 2);
     b.add(&h->steps_bar, 1);
-    b.add(&h->d_status, 1);
     b.add(&h->out, (size_t)NOUT * nodes(h));
     if ((rc = b.commit(&h->blk))) return fail(rc);
   }
   h->stale_dpw = h->stale_dpw2;
-  cudaMemsetAsync(h->d_status, 0, sizeof(int), h->stream);
+  h->d_status = reinterpret_cast<int*>(h->d_kk + 1);
+  cudaMemsetAsync(h->d_kk, 0, 2 * sizeof(long long), h->stream);
   cudaMemsetAsync(h->steps_bar, 0, sizeof(unsigned), h->stream);
   if (h->ring) cudaMemsetAsync(h->ring, 0, rb, h->stream);
   if ((rc = make_tensor_maps(h))) return fail(rc);
@@ -1245,7 +1336,6 @@ int lbm_create(const lbm_params* pin, lbm_sim** out) {
   cudaMemsetAsync(h->f[0], 0, fbytes, h->stream);
   cudaMemsetAsync(h->f[1], 0, fbytes, h->stream);
   cudaMemsetAsync(h->tile_count, 0, sizeof(int) * 2 * ntiles, h->stream);
-  cudaMemsetAsync(h->d_kk, 0, sizeof(long long), h->stream);
   const double inf = INFINITY;
   cudaMemcpyAsync(h->stale_dpw, &inf, sizeof(double), cudaMemcpyHostToDevice, h->stream);
   if ((rc = setup_particle_buffers(h, 0, 0.0))) return fail(rc);
@@ -1313,24 +1403,35 @@ int lbm_step(lbm_sim* h, int32_t nsteps) {
   int st = sticky_status(h);
   if (st) return st;
   cudaSetDevice(h->p.device);
-  for (int32_t s = 0; s < nsteps;) {
+  const long long end = h->kk + nsteps;
+  const bool small = steps_resident(h);
+  bool room = false;
+  for (int32_t s = 0, look = 0; s < nsteps;) {
     int n = 1;
+    if (s >= look) {
+      room = start_running(h, end, small ? h->steps_grid : h->sms);
+      look = s + STEPS_RECHECK;
+    }
     // A call of one step, with tile lists up to date: the two kernels.  k_steps
     // sets itself up at each launch; a call of n steps and the read of the
     // disks, us, k_steps / two kernels, 201 x 601: FP64 n = 1 43.7 / 37.3, n = 2
     // 47.1 / 50.0, n = 4 62.9 / 67.6; FP32 43.3 / 34.2, 45.0 / 45.8, 57.1 / 58.5.
     const bool one = nsteps == 1 && !h->lists_stale;
-    int rc = steps_resident(h) && !one ? enqueue_steps(h, nsteps - s, &n) : enqueue_step(h);
-    if (rc) return rc;
+    const bool resident = small && room && !one;
+    int rc = resident ? enqueue_steps(h, nsteps - s, &n) : enqueue_step(h);
     s += n;
+    if (rc == LBM_OK && resident && s < nsteps) rc = steps_throttle(h);
+    if (rc) {
+      stop_running(h);
+      return rc;
+    }
   }
-  if (h->series) {
-    int rc = series_enqueue(h);  // this call's records, copied behind its kernels
-    if (rc) return rc;
-  }
+  int rc = LBM_OK;
+  if (h->series) rc = series_enqueue(h);  // this call's records, copied behind its kernels
   h->out_kk = -1;
-  CK(cudaMemcpyAsync(h->h_status, h->d_status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-  return LBM_OK;
+  if (rc == LBM_OK) rc = copy_progress(h);
+  if (rc) stop_running(h);
+  return rc;
 }
 
 int lbm_get_step(lbm_sim* h, int64_t* kk) {
@@ -1958,7 +2059,9 @@ extern "C" int lbm_adjoint(lbm_sim* h, const lbm_objective* obj, double* value, 
                                           : std::max<long long>(1, std::llround(std::sqrt((double)N)));
   L = std::max<long long>(1, std::min<long long>(L, std::max<long long>(nlev, 1)));
   const int C = nlev > 0 ? (int)((nlev + L - 1) / L) : 0;
-  const bool resident = adj_resident(h);
+  const bool small = adj_resident(h);
+  RunningScope run(h, small ? h->steps_grid : h->sms);
+  const bool resident = small && run.room;
   const int nsets = C >= 2 && !resident ? 2 : 1;
   int rc = adj_reserve(h, nsets * (int)L, C, N + 1);
   if (rc) return rc;
@@ -2408,6 +2511,7 @@ int lbm_batch_step(lbm_batch* b, int32_t nsteps) {
   int rc;
   int32_t left = nsteps;
   if (left == 0) return LBM_OK;
+  const RunningScope run(b->sims[0], b->sims[0]->sms);  // its kernels fill the GPU
   // a simulation whose force sums are not yet valid (fresh, restarted) takes
   // one step with its own decode flag before the rest can be uniform
   if (b->shape < 0) {

@@ -201,7 +201,13 @@ int lbm_set_particles(lbm_sim* h, int32_t np, const double* pin);
  * C1:241-319 / C6:293-351 / C3:306-399: repulsion, Newton-Euler update,
  * solid fraction, MRT collision, streaming, boundary conditions,
  * macroscopic variables, SPM force field, hydrodynamic force, velocity
- * correction, mean-density check (at history steps). */
+ * correction, mean-density check (at history steps).
+ *
+ * A small lattice takes many steps per kernel launch, unless other handles of
+ * the process run at the same time and would have to take turns with it: then
+ * it takes one launch per kernel, as a large lattice does.  The results are
+ * the same either way.  A call of several thousand steps returns when no more
+ * than about the last two thousand are still to run. */
 int lbm_step(lbm_sim* h, int32_t nsteps);
 
 /* Completed time steps (KK). */
@@ -306,7 +312,9 @@ int32_t lbm_checked_build(void);
  * planes, L = checkpoint_every; a segment's recompute runs on a second
  * stream of the handle beside the reverse sweep of the segment after it (a
  * small lattice takes one set of slots and the segments in turn).
- * The call returns when the sweep is done.
+ * The call returns when the sweep is done.  While other handles of the process
+ * run, a small lattice takes the large one's way; the gradients of the two ways
+ * agree as far as their sums are rounded (the objective to the bit).
  * grads receives 2 + 3*np doubles:
  *   [LBM_GRAD_TAU_Y] dJ/dtau_y   [LBM_GRAD_NU] dJ/dnu (plastic viscosity)
  *   then per disk p: dJ/drho_p, dJ/dx0, dJ/dy0 at LBM_GRAD_HEAD + 3p.
