@@ -49,6 +49,7 @@ struct StepsShared {
   unsigned long long mass;
   double stale;                        // D_PW left by the previous step
   int n, moved, stop;
+  long long kk_stop;                   // the step at which stop was set
 };
 static_assert(STEPS_MAX_DISKS <= 256, "pair lists hold byte indices");
 
@@ -278,17 +279,16 @@ __global__ void __launch_bounds__(STEPS_TPB, 1)
   if (tid == 0) {
     S.stop = timed_out(a.status) ? 1 : 0;
     S.moved = S.n = 0;
+    S.kk_stop = q.kk0;
     S.next = S.next_late = S.n_late = 0;
     S.mass = 0ull;
     S.stale = __ldcg(q.stale + q.stale0);
   }
   __syncthreads();
-  const int nsteps = S.stop ? 0 : q.nsteps;
   if (p.np > 0) steps_lists(p, S, (int)(q.kk0 & 1), row0, row1);
   const bool disk_warp = warp * 32 < p.np;
   if (disk_warp) steps_disk_terms(p, S, q.kk0 + 1);
-  int done = 0;
-  for (int s = 1; s <= nsteps; ++s) {
+  for (int s = 1; s <= q.nsteps && !S.stop; ++s) {
     const long long kk = q.kk0 + s;
     const bool rec = p.series != nullptr && p.series_every > 0 && kk % p.series_every == 0;
     const long long from = (s - 1) & q.mask, to = s & q.mask;
@@ -396,22 +396,23 @@ __global__ void __launch_bounds__(STEPS_TPB, 1)
     // ---- to the next step: the last warp keeps the barrier, the first ones
     //      prepare the disks meanwhile
     __syncthreads();
-    done = s;
-    if (s == nsteps) break;
+    if (s == q.nsteps) break;
     if (tid == STEPS_TPB - 32) {
       S.next = S.next_late = S.n_late = 0;
       grid_arrive(q.bar);
-      if (!grid_wait(q.bar, q.bar0 + (unsigned)s * gridDim.x, a.status)) S.stop = 1;
+      if (!grid_wait(q.bar, q.bar0 + (unsigned)s * gridDim.x, a.status)) {
+        S.stop = 1;
+        S.kk_stop = kk;
+      }
     }
     if (disk_warp) steps_disk_terms(p, S, kk + 1);
     __syncthreads();
-    if (S.stop) break;
   }
   // ---- the state of the last step, into the other copy (a block that starts
   //      late may still be reading the first); after an expired wait too, as
   //      the host goes on with that copy ---------------------------------------
   if (blockIdx.x == 0) {
-    const long long kk = q.kk0 + done;
+    const long long kk = S.stop ? S.kk_stop : q.kk0 + q.nsteps;
     for (int e = tid; e < PS * p.np; e += STEPS_TPB) {
       const int f = e / p.np, id = e - f * p.np;
       const double v = f == P_X || f == P_Y ? S.pos[kk & 1][f == P_X ? 0 : 1][id] : S.rec[f][id];
