@@ -1065,16 +1065,20 @@ int copy_progress(lbm_sim* h) {
   return LBM_OK;
 }
 
-// Between two launches of k_steps in one call: waits until no more than one
-// launch's steps are still to run, so that a call of many steps can give way to
-// a handle that starts meanwhile (the launches of the two kernels hold their
-// caller back in the same way, by the depth of the launch queue).
-int steps_throttle(lbm_sim* h) {
+// Between two launches of k_steps in one call: copies the progress every
+// STEPS_MAX_LAUNCH steps (*mark: the step of the last copy; a copy between two
+// launches costs about 10 us) and waits until the copy before has arrived, so
+// that a call of many steps can give way to a handle that starts meanwhile (the
+// launches of the two kernels hold their caller back in the same way, by the
+// depth of the launch queue).
+int steps_throttle(lbm_sim* h, long long* mark) {
+  if (h->kk - *mark < STEPS_MAX_LAUNCH) return LBM_OK;
+  const long long before = *mark;
+  *mark = h->kk;
   int rc = copy_progress(h);
   if (rc) return rc;
   const auto t0 = std::chrono::steady_clock::now();
-  while (*(volatile long long*)h->h_kk < h->kk - STEPS_MAX_LAUNCH &&
-         *(volatile int*)h->h_status == 0) {
+  while (*(volatile long long*)h->h_kk < before && *(volatile int*)h->h_status == 0) {
     if (std::chrono::steady_clock::now() - t0 > std::chrono::seconds(1)) {
       CK(cudaStreamSynchronize(h->stream));  // or the error that keeps the copy away
       break;
@@ -1404,6 +1408,7 @@ int lbm_step(lbm_sim* h, int32_t nsteps) {
   if (st) return st;
   cudaSetDevice(h->p.device);
   const long long end = h->kk + nsteps;
+  long long mark = h->kk;
   const bool small = steps_resident(h);
   bool room = false;
   for (int32_t s = 0, look = 0; s < nsteps;) {
@@ -1420,7 +1425,7 @@ int lbm_step(lbm_sim* h, int32_t nsteps) {
     const bool resident = small && room && !one;
     int rc = resident ? enqueue_steps(h, nsteps - s, &n) : enqueue_step(h);
     s += n;
-    if (rc == LBM_OK && resident && s < nsteps) rc = steps_throttle(h);
+    if (rc == LBM_OK && resident && s < nsteps) rc = steps_throttle(h, &mark);
     if (rc) {
       stop_running(h);
       return rc;
