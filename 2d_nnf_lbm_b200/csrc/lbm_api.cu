@@ -171,8 +171,12 @@ constexpr int STEPS_RECHECK = 256;      // steps between two looks at the other 
 #define LBM_STEPS_MAX_NODES 400000
 #endif
 constexpr long long STEPS_MAX_NODES = LBM_STEPS_MAX_NODES;
+constexpr long long STEPS_MAX_NODES_F32 = 300000;
 constexpr long long STEPS_NODES_PER_DISK = 700;
+// adjoint: FP32, Bingham FP64, Bingham FP32
 constexpr long long ADJ_LEVELS_MAX_NODES_F32 = 160000;
+constexpr long long ADJ_LEVELS_MAX_NODES_BINGHAM = 70000;
+constexpr long long ADJ_LEVELS_MAX_NODES_BINGHAM_F32 = 90000;
 
 int cuda_fail(cudaError_t e) {
   if (e == cudaErrorMemoryAllocation) return LBM_E_NOMEM;
@@ -975,20 +979,26 @@ int enqueue_step(lbm_sim* h) {
   return LBM_OK;
 }
 
-// Whether the handle steps several steps per launch (k_steps).  The line is
+// Whether the handle may step several steps per launch (k_steps).  The line is
 // where the two ways take about the same time (us per step, k_steps / the
-// particle and step kernels, a record every 10 steps): FP64 201 x 601 7.1 /
-// 9.5, 401 x 801 10.5 / 12.6, 501 x 1001 14.0 / 15.2, Bingham 361 x 1081 17.3 /
-// 18.4; FP32 6.2 / 9.0, 9.0 / 9.8, 11.5 / 11.2, 13.2 / 12.9.  A step of k_steps
-// grows faster with the lattice (its blocks load by node, the step kernel by
-// TMA tiles) and with the disks (each block updates all of them): at 513 x 513
-// with 100 disks 14.5 / 14.7 (FP64) and 12.4 / 13.0, with 200 disks 17.8 / 16.4
-// and 15.1 / 14.4.
+// particle and step kernels, one disk, a record every 10 steps):
+//               201 x 601   301 x 801    401 x 801    361 x 1081   501 x 1001
+//   FP64        7.4 / 9.7    9.7 / 10.6  11.0 / 12.6  12.4 / 13.1  14.3 / 15.1
+//     Bingham   9.8 / 12.0  13.6 / 14.1  15.6 / 18.0  18.2 / 18.1  21.5 / 20.4
+//   FP32        6.5 / 8.6    8.4 / 9.2    9.4 / 9.4   10.6 / 9.9   11.8 / 11.2
+//     Bingham   8.1 / 10.0  10.9 / 11.6  12.4 / 12.1  14.1 / 12.7  15.9 / 13.9
+// (FP32 at 351 x 851, the last size below its line: 8.6 / 9.5, Bingham 11.2 /
+// 12.1).  A step of k_steps grows faster with the lattice (its blocks load by
+// node, the step kernel by TMA tiles) and with the disks (each block updates all
+// of them): at 513 x 513 with 10 / 60 / 140 / 200 disks FP64 11.7 / 11.9, 15.0 /
+// 14.3, 15.2 / 15.2, 16.0 / 16.4; FP32 9.8 / 10.4, 12.3 / 12.1, 12.5 / 12.8,
+// 13.5 / 14.9.
 // A lattice with more row segments than k_steps' queues hold (steps_grid 0)
 // takes the two kernels at any node count.
 bool steps_resident(const lbm_sim* h) {
   return h->steps_grid > 0 && !h->prof && !h->m.bgk && h->np <= STEPS_MAX_DISKS &&
-         nodes(h) + STEPS_NODES_PER_DISK * h->np <= STEPS_MAX_NODES;
+         nodes(h) + STEPS_NODES_PER_DISK * h->np <= STEPS_MAX_NODES &&
+         (h->prec == LBM_FP64 || nodes(h) <= STEPS_MAX_NODES_F32);
 }
 
 // Arguments of a launch of k_steps over the next n steps.  slots: the
@@ -1870,14 +1880,22 @@ int adj_reserve(lbm_sim* h, int nslots, int nck, long long nhist) {
   return LBM_OK;
 }
 
-// Whether an adjoint sweeps many levels per launch (k_adj_levels, with k_steps
-// for the forward pass and the recompute).  us per step of the whole gradient
-// at 200 steps, that way / one launch per kernel: FP64 101 x 301 28.0 / 32.4,
-// 201 x 501 34.7 / 35.3, 301 x 801 47.3 / 54.2, 351 x 1101 58.8 / 64.2; FP32
-// 101 x 301 26.3 / 30.5, 201 x 501 29.8 / 31.9 (Bingham 34.2 / 33.8), 301 x
-// 801 38.9 / 40 (46.4 / 41.9), 351 x 1101 47.8 / 42.8 (65.3 / 47.8).
+// Whether an adjoint may sweep many levels per launch (k_adj_levels, with
+// k_steps for the forward pass and the recompute).  us per step of the whole
+// gradient over 400 steps, that way / one launch per kernel:
+//               101 x 301    255 x 255    201 x 501    201 x 601    301 x 801    351 x 1101
+//   FP64       24.4 / 29.3               33.3 / 33.2  33.0 / 34.7  45.0 / 47.1  58.1 / 64.0
+//     Bingham  28.9 / 32.7  30.1 / 32.8  39.4 / 36.1  40.2 / 39.3  57.7 / 55.1  75.6 / 78.0
+//   FP32       21.8 / 26.8               28.3 / 28.6  28.4 / 29.1  38.4 / 34.1  48.5 / 40.3
+//     Bingham  24.6 / 32.5  25.0 / 29.5  32.3 / 32.1  32.8 / 31.6  45.8 / 39.0  59.8 / 46.2
+// (a Bingham level carries the viscosity's derivative: at 191 x 461 FP64 35.7 /
+// 34.8, FP32 29.6 / 30.5).
 bool adj_resident(const lbm_sim* h) {
-  return steps_resident(h) && (h->prec == LBM_FP64 || nodes(h) <= ADJ_LEVELS_MAX_NODES_F32);
+  const bool f32 = h->prec != LBM_FP64;
+  const long long most = h->m.bingham ? (f32 ? ADJ_LEVELS_MAX_NODES_BINGHAM_F32
+                                             : ADJ_LEVELS_MAX_NODES_BINGHAM)
+                                      : (f32 ? ADJ_LEVELS_MAX_NODES_F32 : STEPS_MAX_NODES);
+  return steps_resident(h) && nodes(h) <= most;
 }
 
 // out[k] = src[k * stride]: one field of one disk's records, every step.
