@@ -2,12 +2,12 @@
 //
 // A small lattice does not fill the GPU for long: 201 x 601 nodes are two
 // passes of one 512-thread block per SM, and what a step takes in kernels of
-// its own (9.5 us FP64, 9.0 us FP32) is the chain of two dependent kernels,
+// its own (9.7 us FP64, 8.6 us FP32) is the chain of two dependent kernels,
 // their start-up and the particle kernel's own latency.  k_steps stays resident over many steps
 // (a cooperative launch, one block per SM): each block owns a contiguous range
 // of 32-node row segments, the populations stay in L2 (17 MB of the 126 MB at
 // that size), and the only synchronisation between blocks is one grid-wide
-// barrier per step.  It takes 7.1 us (FP64) and 6.2 us (FP32): about 2 us the
+// barrier per step.  It takes 7.2 us (FP64) and 6.3 us (FP32): about 2 us the
 // barrier, 1 us the disk's update, the rest the node arithmetic; a history
 // record every step costs 0.6 us more.
 //

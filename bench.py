@@ -32,10 +32,11 @@ Objects of the JSON line beside the headline (N=1; --parts selects them):
 
 --profile-run CASE runs one workload for a few steps with no timing around
 it, for ncu captures of single launches: step-fp32 / step-fp64 (the bench
-workload), visco (the viscoplastic workload at Bn = 2, FP32), adjoint (the
+workload), visco / visco-fp64 (the viscoplastic workload at Bn = 2), adjoint (the
 adjoint workload, objective over the last 100 steps),
 batch (the first --batch-sims runs of the batched workload on the
-TMA-staged batched kernel).
+TMA-staged batched kernel), small (the resident kernel on 201 x 601 and
+101 x 301 nodes).
 
 Multi-GPU: the hot path does not shard (one simulation, one GPU); --gpus N
 runs N independent replicas (weak scaling), timed as the max over ranks.
@@ -96,7 +97,8 @@ def parse_args(argv=None):
     ap.add_argument("--ny", type=int, default=2048)
     ap.add_argument("--particles", type=int, default=512)
     ap.add_argument("--profile-run", default="",
-                    choices=["", "step-fp32", "step-fp64", "visco", "adjoint", "batch"])
+                    choices=["", "step-fp32", "step-fp64", "visco", "visco-fp64", "adjoint", "batch",
+                             "small"])
     a = ap.parse_args(argv)
     parts = set(PARTS) if a.parts == "all" else {s.strip() for s in a.parts.split(",") if s.strip()}
     unknown = parts - set(PARTS)
@@ -901,8 +903,20 @@ def profile_run(pkg, args):
               f"status {max(abs(s.status()) for s in b.sims)}")
         b.close()
         return 0
-    if args.profile_run == "visco":
-        p, pin, _ = pkg.cases.workload_cfg3(1, 2.0)
+    if args.profile_run == "small":  # 201 x 601 and 101 x 301: the resident kernel
+        for nx, ny in ((200, 600), (100, 300)):
+            p = pkg.cases.shipped_c1(nx, ny, 24.0)
+            p.series_every = 0
+            with pkg.Simulation(p) as sim:
+                sim.set_particles(pkg.cases.pin_array([[nx / 2, 0.75 * ny]], 24.0, 1.25))
+                for n in (2, args.steps):
+                    sim.step(n)
+                parts = sim.particles()
+                print(f"steps {sim.kk}  disk at ({parts[0, 0]:.6f}, {parts[0, 1]:.6f})  "
+                      f"status {sim.status()}")
+        return 0
+    if args.profile_run in ("visco", "visco-fp64"):
+        p, pin, _ = pkg.cases.workload_cfg3(1 if args.profile_run == "visco" else 0, 2.0)
         with pkg.Simulation(p) as sim:
             sim.set_particles(pin)
             sim.step(args.steps)
