@@ -204,7 +204,7 @@ int lbm_set_particles(lbm_sim* h, int32_t np, const double* pin);
  * correction, mean-density check (at history steps).
  *
  * A small lattice takes many steps per kernel launch, unless other handles of
- * the process run at the same time and would have to take turns with it: then
+ * the process run at the same time and would have to wait for it: then
  * it takes one launch per kernel, as a large lattice does.  The results are
  * the same either way.  A launch of many steps keeps its SMs to itself (all of
  * them, from a few ten thousand nodes) for up to 1024 steps, several
