@@ -2101,9 +2101,15 @@ extern "C" int lbm_adjoint(lbm_sim* h, const lbm_objective* obj, double* value, 
   const int C = nlev > 0 ? (int)((nlev + L - 1) / L) : 0;
   const bool small = adj_resident(h);
   RunningScope run(h, small ? h->steps_grid : h->sms);
-  const bool resident = small && run.room;
+  bool resident = small && run.room;
   const int nsets = C >= 2 && !resident ? 2 : 1;
   int rc = adj_reserve(h, nsets * (int)L, C, N + 1);
+  if (rc == LBM_E_NOMEM && nsets == 2 && steps_resident(h)) {
+    // the second slot set does not fit: a lattice that can do without it does
+    cudaGetLastError();
+    resident = true;
+    rc = adj_reserve(h, (int)L, C, N + 1);
+  }
   if (rc) return rc;
   const size_t rec = (size_t)PS * h->npad;
   const size_t sb = adj_slot_bytes(h);

@@ -51,3 +51,34 @@ def test_gradients_at_the_line(pkg, cases, program, nx, ny, prec):
             a, b = np.atleast_1d(g[k]), np.atleast_1d(gr[k])
             assert np.all(np.isfinite(a)), k
             assert np.all(np.abs(a - b) <= rtol * (np.abs(b) + scale)), (k, a, b)
+
+
+def test_gradient_that_fits_one_slot_set_only(pkg, cases):
+    """Above the line a gradient keeps two sets of slots; a lattice that can
+    step many steps per launch takes the one-set way where the second set does
+    not fit in memory, and returns the same gradient (2e-9)."""
+    torch = pytest.importorskip("torch")
+    p, pin = build(cases, "c6", 280, 280, 2, 20.0, 0)
+    p.contact_test, p.series_every = 0, 0
+    every, n1 = 200, 404  # three segments; a slot is 10 planes of 281 rows
+    want = run(pkg, p, pin, 400, n1, every, False)
+    slot = 10 * 281 * 288 * 8
+    sim = pkg.Simulation(p)
+    sim.set_particles(pin)
+    free, _ = torch.cuda.mem_get_info()
+    taken = torch.empty(free - int(1.5 * every * slot) - (64 << 20), dtype=torch.uint8,
+                        device="cuda")
+    try:
+        j, g = sim.adjoint(400, n1, particle=1, checkpoint_every=every)
+        parts = sim.particles()
+    finally:
+        del taken
+        torch.cuda.empty_cache()
+    assert sim.status() == 0
+    sim.close()
+    assert j == want[0] and np.array_equal(parts, want[2])
+    for k, w in want[1].items():
+        a, b = np.atleast_1d(g[k]), np.atleast_1d(w)
+        scale = np.max(np.abs(b)) if k not in ("x0", "y0") else max(
+            np.max(np.abs(want[1]["x0"])), np.max(np.abs(want[1]["y0"])))
+        assert np.all(np.abs(a - b) <= 2e-9 * (np.abs(b) + scale)), k
