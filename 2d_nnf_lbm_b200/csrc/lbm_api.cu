@@ -1854,6 +1854,8 @@ int adj_reserve(lbm_sim* h, int nslots, int nck, long long nhist) {
   if (nck > h->adj_nck || h->adj_npad != h->npad) {
     dfree(h->adj_ck);
     dfree(h->adj_ckp);
+    h->adj_ck = nullptr;  // none is allocated for a gradient without levels
+    h->adj_ckp = nullptr;
     h->adj_nck = 0;
     if (nck > 0 && (rc = dalloc(&h->adj_ck, sb * nck))) return rc;
     if ((rc = dalloc(&h->adj_ckp, adj_ckp_len(h) * (nck + 1)))) return rc;
