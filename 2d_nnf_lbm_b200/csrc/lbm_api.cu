@@ -198,6 +198,7 @@ int dalloc(T** p, size_t count) {
   if (count == 0) count = 1;
   cudaError_t e = cudaMalloc(reinterpret_cast<void**>(p), count * sizeof(T));
   if (e != cudaSuccess) {
+    cudaGetLastError();  // reported here, not by the next launch's check
     *p = nullptr;
     return cuda_fail(e);
   }
@@ -2108,7 +2109,6 @@ extern "C" int lbm_adjoint(lbm_sim* h, const lbm_objective* obj, double* value, 
   int rc = adj_reserve(h, nsets * (int)L, C, N + 1);
   if (rc == LBM_E_NOMEM && nsets == 2 && steps_resident(h)) {
     // the second slot set does not fit: a lattice that can do without it does
-    cudaGetLastError();
     resident = true;
     rc = adj_reserve(h, (int)L, C, N + 1);
   }

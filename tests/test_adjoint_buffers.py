@@ -37,3 +37,28 @@ def test_gradient_without_levels_after_one_with(pkg, cases):
         o.close()
     for m in more:
         m.close()
+
+
+def test_refused_allocation_leaves_no_error_behind(pkg, cases):
+    """A gradient that does not fit in memory is LBM_E_NOMEM, and the calls
+    after it are not."""
+    torch = pytest.importorskip("torch")
+    p, pin = build(cases, "c6", 280, 280, 2, 20.0, 0)
+    p.contact_test, p.series_every = 0, 0
+    s = pkg.Simulation(p)
+    s.set_particles(pin)
+    before = s.particles()
+    free, _ = torch.cuda.mem_get_info()
+    taken = torch.empty(free - (256 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        with pytest.raises(pkg.LbmError) as err:
+            s.adjoint(400, 404, checkpoint_every=200)
+        assert err.value.code == -3  # LBM_E_NOMEM
+        assert np.array_equal(s.particles(), before)
+        assert np.isfinite(s.field("ux")).all() and s.status() == 0
+    finally:
+        del taken
+        torch.cuda.empty_cache()
+    s.step(10)
+    assert s.status() == 0 and s.kk == 10
+    s.close()
